@@ -18,6 +18,8 @@
 //                      bit-identical to hostLevinLaplacian (Matting.cu:39-219).
 #include <string.h>
 
+#include <type_traits>
+
 #include "gm_internal.cuh"
 
 int gm_note_status(int s);
@@ -104,107 +106,329 @@ struct SymOut {
     float* a25;       // optional [25][apitch]
     size_t apitch;
     float* b25;       // optional [N]
+    float* d;         // [H][pitch] gamma + row sum of w
+    float* d32;       // [H][pitch] gamma + row sum of w32; NULL: 25 bands only (w, w32, gamma, b, d unset)
 };
 
-template <class T>
-__global__ void __launch_bounds__(TW * TH) levin_sym_kernel(ImgView im, ScribView sc, double eps, int W, int H,
-                                                            SymOut o)
+// ---- FP64 assembly: one streaming pass over the image ----
+//
+// With S = sum of a window's 9 colours, D_i = 9 x_i - S and
+// N = 9 sum(x x^T) - S S^T = 81 Sigma, a window's term of the pair (i, j) is
+//     (1 + (x_i - mu)^T (Sigma + eps/9 I)^-1 (x_j - mu)) / 9
+//         = (1 + e_i . D_j) / 9,     e_i = (N + 9 eps I)^-1 D_i,
+// one solve per pixel of the window and one 3-vector product per pair: about
+// 340 FP64 operations per pixel of the image (24 neighbours of 9 windows each
+// on their own, with an FP64 division each, took 1,500).  Only the 12 upper
+// couplings are formed.  Colours of an RGB8 image stay whole numbers
+// (x = 0..255, eps scaled by 255^2), so S, N and D are exact.
+//
+// Thread t of a CTA owns the windows centred on column u0 - 1 + t and marches
+// down the rows with the 9 colours of its window in registers.  Sums over the
+// vertically neighbouring windows stay in registers; the horizontal ones
+// (3 - |du| windows per pair) take 9 values per row through shared memory.
+// The thread of column u finishes the couplings with du = -1, 0, 1 of pixel u,
+// du = 2 of pixel u - 1 and du = -2 of pixel u + 1 (one window column only).
+// The rounded couplings go through a ring in shared memory, from which the
+// diagonal (the sum of exactly the stored weights) is formed in the same pass
+// instead of in a second one that reads all planes again (84 B/px).  The first
+// rows of a run repeat the couplings of the two rows above it; runs are as
+// long as one wave of CTAs allows.
+//
+// Measured with the FP16 store: 1080p RGB8 450 -> 122 us, 4096^2 870 us (83 B
+// written per pixel are 26 and 215 us); FP32 store, 4001 x 2999: 2,400 -> 540
+// (RGB8), 620 us (float).  Bound by instruction issue at 12 warps per SM (59 %
+// of the slots, FP64 pipe 37 %); a first form that kept the windows in shared
+// memory took 156 us, bound by its reads (12 shared wavefronts per 32 pixels
+// and window).
+constexpr int kAT = 128;              // threads = window columns
+constexpr int kAW = kAT - 2;          // output columns per CTA
+constexpr int kAP = kAT + 4;          // row length in shared memory (two pad columns each side)
+// CTAs per SM the registers are cut for.  A float image's 27 colours and 18 row
+// sums in 64 bits spill at 168 registers (1080p: 160 us with 3 CTAs per SM, 135
+// with 2); an RGB8 image's do not (122 us with 3, 135 with 2).
+__host__ __device__ constexpr int asm_ctas(bool f32) { return f32 ? 2 : 3; }
+constexpr int kMinRows = 2;
+
+// Rows of the coupling ring: couplings to the same row are read in the step
+// that forms them, those to the next row one step later, to the second row
+// two steps later.
+__host__ __device__ constexpr int ring_base(int k) { return k <= 2 ? k - 1 : (k <= 7 ? 2 + 2 * (k - 3) : 12 + 3 * (k - 8)); }
+__host__ __device__ constexpr int ring_len(int k) { return k <= 2 ? 1 : (k <= 7 ? 2 : 3); }
+constexpr int kRingRows = 27;
+
+// |n| < 2^31, given as n + 2^31, to double with one FP64 addition (the
+// conversion instruction runs at a quarter of the FP64 rate).
+__device__ __forceinline__ double biased_to_double(unsigned n)
 {
-    __shared__ double col[TH + 4][TW + 4][3];
-    __shared__ double wmu[NWIN][3];
-    __shared__ double wki[NWIN][6];  // inverse covariance: 00 01 02 11 12 22
-    const int u0 = blockIdx.x * TW, v0 = blockIdx.y * TH;
-    const int tid = threadIdx.x;
-    for (int t = tid; t < (TH + 4) * (TW + 4); t += blockDim.x) {
-        const int x = t % (TW + 4), y = t / (TW + 4);
-        const int u = u0 - 2 + x, v = v0 - 2 + y;
-        double r = 0, g = 0, b = 0;
-        if (u >= 0 && u < W && v >= 0 && v < H) load_rgb_d(im, u, v, r, g, b);
-        col[y][x][0] = r; col[y][x][1] = g; col[y][x][2] = b;
+    return __hiloint2double(0x43300000, (int)n) - 4503601774854144.0;  // 2^52 + 2^31
+}
+
+template <class T, bool F32IMG, bool BANDS>
+__global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgView im, ScribView sc, double e9, int W, int H,
+                                                                       int rows, SymOut o)
+{
+    constexpr bool kLow = sizeof(T) == 2;
+    using Sum = typename std::conditional<F32IMG, double, int>::type;
+    using Pix = typename std::conditional<F32IMG, float, int>::type;
+    __shared__ double xch[9][kAP];
+    __shared__ float hi[kRingRows][kAP];
+    __shared__ T lo[kLow ? kRingRows : 1][kAP];
+    const int t = threadIdx.x, c = t + 2, u = blockIdx.x * kAW - 1 + t;
+    const int r0 = blockIdx.y * rows, r1 = min(r0 + rows, H), rs0 = max(r0 - 2, 0);
+    const bool ok_col = u >= 1 && u <= W - 2;
+    for (int i = t; i < kRingRows * kAP; i += kAT) {
+        hi[i / kAP][i % kAP] = 0.f;
+        if (kLow) lo[i / kAP][i % kAP] = T(0.f);
     }
-    __syncthreads();
-    for (int t = tid; t < NWIN; t += blockDim.x) {
-        const int wx = t % (TW + 2), wy = t / (TW + 2);
-        const int cu = u0 - 1 + wx, cv = v0 - 1 + wy;
-        if (cu < 1 || cu > W - 2 || cv < 1 || cv > H - 2) continue;
-        double m[3] = {0, 0, 0}, c[6] = {0, 0, 0, 0, 0, 0};
-        for (int q = 0; q < 9; ++q) {
-            const double* p = col[wy + q / 3][wx + q % 3];
-            m[0] += p[0]; m[1] += p[1]; m[2] += p[2];
-            c[0] += p[0] * p[0]; c[1] += p[0] * p[1]; c[2] += p[0] * p[2];
-            c[3] += p[1] * p[1]; c[4] += p[1] * p[2]; c[5] += p[2] * p[2];
-        }
-        for (int a = 0; a < 3; ++a) m[a] /= 9.0;
-        const double e9 = eps / 9.0;
-        const double s00 = c[0] / 9.0 - m[0] * m[0] + e9, s01 = c[1] / 9.0 - m[0] * m[1],
-                     s02 = c[2] / 9.0 - m[0] * m[2], s11 = c[3] / 9.0 - m[1] * m[1] + e9,
-                     s12 = c[4] / 9.0 - m[1] * m[2], s22 = c[5] / 9.0 - m[2] * m[2] + e9;
-        const double a00 = s11 * s22 - s12 * s12, a01 = s02 * s12 - s01 * s22, a02 = s01 * s12 - s02 * s11;
-        const double a11 = s00 * s22 - s02 * s02, a12 = s02 * s01 - s00 * s12, a22 = s00 * s11 - s01 * s01;
-        const double det = s00 * a00 + s01 * a01 + s02 * a02;
-        const double id = 1.0 / det;
-        wmu[t][0] = m[0]; wmu[t][1] = m[1]; wmu[t][2] = m[2];
-        wki[t][0] = a00 * id; wki[t][1] = a01 * id; wki[t][2] = a02 * id;
-        wki[t][3] = a11 * id; wki[t][4] = a12 * id; wki[t][5] = a22 * id;
-    }
-    __syncthreads();
-    const int lx = tid % TW, ly = tid / TW;
-    const int u = u0 + lx, v = v0 + ly;
-    if (u >= W || v >= H) return;
-    double acc[25];
+
+    // Colours (u - 1, u, u + 1) of row v, zero outside the image (and in an
+    // image without any window, whatever its colours hold).
+    const bool in[3] = {u >= 1 && u <= W, u >= 0 && u < W, u >= -1 && u < W - 1};
+    const bool any = W >= 3 && H >= 3;
+    auto fetch = [&](int v, Pix (&p)[9]) {
 #pragma unroll
-    for (int k = 0; k < 25; ++k) acc[k] = 0.0;
-    const double* xi = col[ly + 2][lx + 2];
+        for (int q = 0; q < 9; ++q) p[q] = 0;
+        if (any && v >= 0 && v < H) {
+            const unsigned char* row = im.data + (size_t)v * im.pitch;
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy) {
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-            const int cu = u + dx, cv = v + dy;
-            if (cu < 1 || cu > W - 2 || cv < 1 || cv > H - 2) continue;
-            const int t = (ly + 1 + dy) * (TW + 2) + (lx + 1 + dx);
-            const double* mu = wmu[t];
-            const double* k = wki[t];
-            const double x0 = xi[0] - mu[0], x1 = xi[1] - mu[1], x2 = xi[2] - mu[2];
-            const double w0 = k[0] * x0 + k[1] * x1 + k[2] * x2;
-            const double w1 = k[1] * x0 + k[3] * x1 + k[4] * x2;
-            const double w2 = k[2] * x0 + k[4] * x1 + k[5] * x2;
-#pragma unroll
-            for (int qy = -1; qy <= 1; ++qy) {
-#pragma unroll
-                for (int qx = -1; qx <= 1; ++qx) {
-                    const int ju = dx + qx, jv = dy + qy;  // neighbour offset from i
-                    if (ju == 0 && jv == 0) continue;
-                    const double* xj = col[ly + 2 + jv][lx + 2 + ju];
-                    const double t2 = (1.0 + w0 * (xj[0] - mu[0]) + w1 * (xj[1] - mu[1]) + w2 * (xj[2] - mu[2])) / 9.0;
-                    acc[12 + ju + 5 * jv] += t2;
+            for (int b = 0; b < 3; ++b)
+                if (in[b]) {
+                    if constexpr (F32IMG) {
+                        const float4 q = reinterpret_cast<const float4*>(row)[u - 1 + b];
+                        p[3 * b] = q.x; p[3 * b + 1] = q.y; p[3 * b + 2] = q.z;
+                    } else {
+                        const unsigned char* q = row + 3 * (ptrdiff_t)(u - 1 + b);
+                        p[3 * b] = q[0]; p[3 * b + 1] = q[1]; p[3 * b + 2] = q[2];
+                    }
                 }
+        }
+    };
+    // Row sums of the three colours and their six products.
+    auto row_sums = [&](const Pix (&p)[9], Sum (&s)[9]) {
+        int n = 3;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            s[a] = (Sum)p[a] + (Sum)p[3 + a] + (Sum)p[6 + a];
+#pragma unroll
+            for (int b = a; b < 3; ++b, ++n)
+                s[n] = (Sum)p[a] * (Sum)p[b] + (Sum)p[3 + a] * (Sum)p[3 + b] + (Sum)p[6 + a] * (Sum)p[6 + b];
+        }
+    };
+
+    Pix pa[9], pb[9], pc[9], pn[9];  // rows v - 1, v, v + 1 of the window, and the one after
+    Sum sa[9], sb[9], sn[9];         // row sums of rows v - 1 and v
+    fetch(rs0 - 2, pa);
+    fetch(rs0 - 1, pb);
+    fetch(rs0, pc);
+    row_sums(pa, sa);
+    row_sums(pb, sb);
+    // Sums over the windows so far: rows v -> v + 1 (9 pairs of columns) and
+    // within rows v and v + 1 (column pairs 01, 02, 12).
+    double dn1[9], in0[3], in1[3];
+#pragma unroll
+    for (int n = 0; n < 9; ++n) dn1[n] = 0.0;
+#pragma unroll
+    for (int n = 0; n < 3; ++n) in0[n] = in1[n] = 0.0;
+    const size_t plane = o.plane;
+    T* wl = reinterpret_cast<T*>(o.w);
+    const bool own_w = o.w != (void*)o.w32;  // an FP32 store may keep w apart from w32
+    // Output columns: [first, first + kAW) of the image.
+    const int first = blockIdx.x * kAW, last = min(first + kAW, W) - 1;
+    const bool out_col = u >= first && u <= last;
+    __syncthreads();
+
+#pragma unroll F32IMG ? 1 : 2
+    for (int v = rs0 - 1; v <= r1; ++v) {  // window centre row; finishes pixel row r = v - 1
+        const int r = v - 1;
+        fetch(v + 2, pn);
+        const bool out = out_col && r >= r0;
+        // the scribble's raw values, looked at only when the row is done
+        float sc_g = 0.f, sc_s = 0.f;
+        unsigned char sc_m = 128;
+        if (out) {
+            if (sc.gamma_map) {
+                sc_g = sc.gamma_map[(size_t)r * W + u];
+                if (sc.s_map) sc_s = sc.s_map[(size_t)r * W + u];
+            } else if (sc.map) {
+                sc_m = sc.map[(size_t)r * sc.map_pitch + u];
             }
         }
-    }
-    float gam, bv;
-    scribble(sc, u, v, gam, bv);
-    const size_t plane = o.plane;
-    const size_t gi = (size_t)v * o.pitch + u;
-    T* wl = reinterpret_cast<T*>(o.w);
+        row_sums(pc, sn);
+        // --- window statistics and the factors of N + e9 I = L diag(d) L^T
+        // (the error of a solve with them grows with the condition number,
+        // that of the cofactors' inverse with its square); two divisions give
+        // the three 1 / d.
+        const bool ok = ok_col && v >= 1 && v <= H - 2;
+        Sum s[9];
 #pragma unroll
-    for (int k = 1; k <= 12; ++k) {
-        wl[(size_t)(k - 1) * plane + gi] = from_double<T>(acc[12 + k]);
-        o.w32[(size_t)(k - 1) * plane + gi] = __double2float_rn(acc[12 + k]);
-    }
-    o.gamma[gi] = gam;
-    o.b[gi] = bv;
-    if (o.a25) {
-        const size_t i = (size_t)v * W + u;
-        double rs = 0.0;
-#pragma unroll
-        for (int k = 0; k < 25; ++k) {
-            if (k == 12) continue;
-            const float a = __double2float_rn(-acc[k]);
-            o.a25[(size_t)k * o.apitch + i] = a;
-            rs -= (double)a;
+        for (int n = 0; n < 9; ++n) s[n] = sa[n] + sb[n] + sn[n];
+        double N[6];
+        if constexpr (F32IMG) {
+            N[0] = fma(-s[0], s[0], 9.0 * s[3]); N[1] = fma(-s[0], s[1], 9.0 * s[4]); N[2] = fma(-s[0], s[2], 9.0 * s[5]);
+            N[3] = fma(-s[1], s[1], 9.0 * s[6]); N[4] = fma(-s[1], s[2], 9.0 * s[7]); N[5] = fma(-s[2], s[2], 9.0 * s[8]);
+        } else {
+            const unsigned B = 0x80000000u;
+            N[0] = biased_to_double(9 * s[3] - s[0] * s[0] + B); N[1] = biased_to_double(9 * s[4] - s[0] * s[1] + B);
+            N[2] = biased_to_double(9 * s[5] - s[0] * s[2] + B); N[3] = biased_to_double(9 * s[6] - s[1] * s[1] + B);
+            N[4] = biased_to_double(9 * s[7] - s[1] * s[2] + B); N[5] = biased_to_double(9 * s[8] - s[2] * s[2] + B);
         }
-        o.a25[(size_t)12 * o.apitch + i] = __double2float_rn(rs + (double)gam);
-        if (o.b25) o.b25[i] = bv;
+        const double s00 = N[0] + e9, s11 = N[3] + e9, s22 = N[5] + e9;
+        const double c22 = fma(s00, s11, -N[1] * N[1]), c12 = fma(s00, N[4], -N[2] * N[1]),
+                     c11 = fma(s00, s22, -N[2] * N[2]);
+        const double ri = 1.0 / (s00 * c22), rc = ri * s00;  // 1 / c22 = rc
+        const double i0 = ok ? ri * c22 : 0.0, i1 = ok ? s00 * rc : 0.0;
+        const double l1 = ok ? N[1] * i0 : 0.0, l2 = ok ? N[2] * i0 : 0.0, l3 = ok ? c12 * rc : 0.0;
+        const double i2 = ok ? s00 * (1.0 / fma(-c12, l3, c11)) : 0.0;
+        const double one = ok ? 1.0 : 0.0;
+        auto dev = [&](const Pix (&p)[9], int b, double (&d)[3]) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                if constexpr (F32IMG) d[a] = fma(9.0, (double)p[3 * b + a], -s[a]);
+                else d[a] = biased_to_double(9u * (unsigned)p[3 * b + a] + (0x80000000u - (unsigned)s[a]));
+            }
+        };
+        auto solve = [&](const double (&d)[3], double (&e)[3]) {
+            const double z1 = fma(-l1, d[0], d[1]), z2 = fma(-l3, z1, fma(-l2, d[0], d[2]));
+            e[2] = i2 * z2;
+            e[1] = fma(i1, z1, -l3 * e[2]);
+            e[0] = fma(i0, d[0], -fma(l1, e[1], l2 * e[2]));
+        };
+        auto pair = [](double acc, const double (&e)[3], const double (&d)[3]) {
+            return fma(e[0], d[0], fma(e[1], d[1], fma(e[2], d[2], acc)));
+        };
+        double da[3][3], db[3][3], dc[3][3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            dev(pa, b, da[b]);
+            dev(pb, b, db[b]);
+            dev(pc, b, dc[b]);
+        }
+        // --- pairs whose upper pixel is in row r: their last window
+        double p2[9], p1[9], p0[3], e[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            solve(da[a], e);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                p2[3 * a + b] = pair(one, e, dc[b]);
+                p1[3 * a + b] = pair(dn1[3 * a + b] + one, e, db[b]);
+            }
+            if (a == 0) {
+                p0[0] = pair(in0[0] + one, e, da[1]);
+                p0[1] = pair(in0[1] + one, e, da[2]);
+            }
+            if (a == 1) p0[2] = pair(in0[2] + one, e, da[2]);
+        }
+        // shares of the neighbouring columns' couplings: [9] planes, read from
+        // t - 1 (0, 1, 4, 5) or t + 1 (2, 3, 6, 7, 8)
+        xch[0][c] = p2[8]; xch[1][c] = p2[7]; xch[2][c] = p2[0]; xch[3][c] = p2[1];
+        xch[4][c] = p1[8]; xch[5][c] = p1[7]; xch[6][c] = p1[0]; xch[7][c] = p1[1];
+        xch[8][c] = p0[0];
+        // --- pairs whose upper pixel is in row v or v + 1: sums to go on with
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            solve(db[a], e);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) dn1[3 * a + b] = pair(one, e, dc[b]);
+            if (a == 0) {
+                in0[0] = pair(in1[0] + one, e, db[1]);
+                in0[1] = pair(in1[1] + one, e, db[2]);
+            }
+            if (a == 1) in0[2] = pair(in1[2] + one, e, db[2]);
+        }
+        solve(dc[0], e);
+        in1[0] = pair(one, e, dc[1]);
+        in1[1] = pair(one, e, dc[2]);
+        solve(dc[1], e);
+        in1[2] = pair(one, e, dc[2]);
+#pragma unroll
+        for (int n = 0; n < 9; ++n) {
+            pa[n] = pb[n]; pb[n] = pc[n]; pc[n] = pn[n];
+            sa[n] = sb[n]; sb[n] = sn[n];
+        }
+        if (r < rs0) continue;
+        __syncthreads();
+        // --- finish the couplings of row r
+        double su = 0.0, su32 = 0.0;  // this pixel's own upper couplings, as rounded
+        const int r2 = r & 1, r3 = r % 3;
+        const bool row_out = r >= r0 && o.w32 != nullptr;
+        const bool st[3] = {row_out && u > first && u <= last + 1, row_out && out_col, row_out && u >= first - 1 && u < last};
+        float* w32 = o.w32 + (size_t)r * o.pitch + u;
+        T* wlo = wl + (size_t)r * o.pitch + u;
+        auto finish = [&](int k, int x, double w9) {  // x: pixel column less u
+            const double w = w9 * (1.0 / 9.0);
+            const float wf = __double2float_rn(w);
+            const int row = ring_base(k) + (ring_len(k) == 1 ? 0 : (ring_len(k) == 2 ? r2 : r3));
+            hi[row][c + x] = wf;
+            if (x == 0) su32 += (double)wf;
+            if (st[x + 1]) w32[(size_t)(k - 1) * plane + x] = wf;
+            if (kLow) {
+                const T wt = from_double<T>(w);
+                lo[row][c + x] = wt;
+                if (x == 0) su += (double)Cvt<T>::to_f(wt);
+                if (st[x + 1]) wlo[(size_t)(k - 1) * plane + x] = wt;
+            } else if (own_w && st[x + 1]) {
+                wlo[(size_t)(k - 1) * plane + x] = from_double<T>(w);
+            }
+        };
+        finish(10, 0, xch[0][c - 1] + p2[4] + xch[2][c + 1]);
+        finish(9, 0, xch[1][c - 1] + p2[3]);
+        finish(11, 0, p2[5] + xch[3][c + 1]);
+        finish(12, -1, p2[2]);
+        finish(8, 1, p2[6]);
+        finish(5, 0, xch[4][c - 1] + p1[4] + xch[6][c + 1]);
+        finish(4, 0, xch[5][c - 1] + p1[3]);
+        finish(6, 0, p1[5] + xch[7][c + 1]);
+        finish(7, -1, p1[2]);
+        finish(3, 1, p1[6]);
+        finish(1, 0, p0[2] + xch[8][c + 1]);
+        finish(2, -1, p0[1]);
+        __syncthreads();
+        // --- diagonal of row r from the rounded couplings
+        if (out) {
+            const size_t gi = (size_t)r * o.pitch + u;
+            // Matting.cu:205-216: 255 -> (gamma, b = gamma), 0 -> (gamma, b = 0)
+            const bool mark = sc_m == 255 || sc_m == 0;
+            const float gam = sc.gamma_map ? sc_g : (mark ? sc.gamma_value : 0.f);
+            const float bv = sc.gamma_map ? (sc.s_map ? sc_g * sc_s : 0.f) : (sc_m == 255 ? sc.gamma_value : 0.f);
+            double s1 = (double)gam + su, s32 = (double)gam + su32;
+            const int r2b = r2 ^ 1, r3b = r3 == 2 ? 0 : r3 + 1;  // rows r - 1 (mod 2), r - 2 (mod 3)
+            float below[13];
+#pragma unroll
+            for (int k = 1; k <= 12; ++k) {
+                const int dv = (k + 2) / 5, du = k - 5 * dv;
+                const int up = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2 : r3));
+                const int dn = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2b : r3b));
+                if (du == 2 || du == -2) s32 += (double)hi[up][c];
+                s32 += (double)hi[dn][c - du];
+                if (kLow) {
+                    if (du == 2 || du == -2) s1 += (double)Cvt<T>::to_f(lo[up][c]);
+                    s1 += (double)Cvt<T>::to_f(lo[dn][c - du]);
+                }
+                if (BANDS) below[k] = hi[dn][c - du];
+            }
+            if (o.d32) {
+                o.gamma[gi] = gam;
+                o.b[gi] = bv;
+                o.d[gi] = __double2float_rn(kLow ? s1 : s32);
+                o.d32[gi] = __double2float_rn(s32);
+            }
+            if (BANDS) {
+                const size_t i = (size_t)r * W + u;
+                double rs = 0.0;
+#pragma unroll
+                for (int k = -12; k <= 12; ++k) {
+                    if (k == 0) continue;
+                    const int ka = k < 0 ? -k : k;
+                    const int up = ring_base(ka) + (ring_len(ka) == 1 ? 0 : (ring_len(ka) == 2 ? r2 : r3));
+                    const float a = -(k < 0 ? below[ka] : hi[up][c]);
+                    o.a25[(size_t)(12 + k) * o.apitch + i] = a;
+                    rs -= (double)a;
+                }
+                o.a25[(size_t)12 * o.apitch + i] = __double2float_rn(rs + (double)gam);
+                if (o.b25) o.b25[i] = bv;
+            }
+        }
     }
 }
 
@@ -355,15 +579,30 @@ __global__ void levin_diag_kernel(const T* __restrict__ w, const float* __restri
     d32[i] = __double2float_rn(s32);
 }
 
-template <class T>
-static void launch_sym(const ImgView& im, const ScribView& sc, double eps, int W, int H, const SymOut& o,
-                       float* d, float* d32, cudaStream_t st)
+template <class T, bool F32IMG, bool BANDS>
+static int launch_sym3(const ImgView& im, const ScribView& sc, double eps, int W, int H, const SymOut& o, int sms,
+                       cudaStream_t st)
 {
-    dim3 grid((W + TW - 1) / TW, (H + TH - 1) / TH);
-    levin_sym_kernel<T><<<grid, TW * TH, 0, st>>>(im, sc, eps, W, H, o);
-    dim3 g2((W + 127) / 128, H);
-    levin_diag_kernel<T><<<g2, 128, 0, st>>>(reinterpret_cast<const T*>(o.w), o.w32, o.gamma, d, d32, W, H, o.pitch,
-                                             o.plane);
+    // One wave: every CTA that fits the GPU gets a run of rows of one strip.
+    const int strips = (W + kAW - 1) / kAW;
+    const int runs = max(1, asm_ctas(F32IMG) * sms / strips);
+    const int rows = max(kMinRows, (H + runs - 1) / runs);
+    const dim3 grid(strips, (H + rows - 1) / rows);
+    const double e9 = 9.0 * eps * (F32IMG ? 1.0 : 255.0 * 255.0);
+    levin_sym_kernel<T, F32IMG, BANDS><<<grid, kAT, 0, st>>>(im, sc, e9, W, H, rows, o);
+    GM_CUDA_TRY(cudaGetLastError());
+    return GM_OK;
+}
+
+template <class T>
+static int launch_sym(const ImgView& im, const ScribView& sc, double eps, int W, int H, const SymOut& o, int sms,
+                      cudaStream_t st)
+{
+    if (im.format == GM_IMAGE_RGBA32F)
+        return o.a25 ? launch_sym3<T, true, true>(im, sc, eps, W, H, o, sms, st)
+                     : launch_sym3<T, true, false>(im, sc, eps, W, H, o, sms, st);
+    return o.a25 ? launch_sym3<T, false, true>(im, sc, eps, W, H, o, sms, st)
+                 : launch_sym3<T, false, false>(im, sc, eps, W, H, o, sms, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -648,7 +887,8 @@ extern "C" int gm_levin_assemble(gm_levin_store* st, const gm_image* im, const g
         return GM_ERR_INVALID;
     }
     if (!(eps >= 0.0)) { gm_set_error_msg("eps must be >= 0"); return GM_ERR_INVALID; }
-    GM_TRY(gm_check_device(nullptr));
+    int sms = 0;
+    GM_TRY(gm_check_device(&sms));
     ImgView iv;
     ScribView sv;
     GM_TRY(make_views(im, sc, st->W, iv, sv));
@@ -658,6 +898,8 @@ extern "C" int gm_levin_assemble(gm_levin_store* st, const gm_image* im, const g
     o.w32 = st->w32;
     o.gamma = st->gamma;
     o.b = st->b;
+    o.d = st->d;
+    o.d32 = st->d32;
     o.pitch = st->pitch;
     o.plane = st->plane_stride ? st->plane_stride : (size_t)st->H * st->pitch;
     if (bands25) {
@@ -671,11 +913,9 @@ extern "C" int gm_levin_assemble(gm_levin_store* st, const gm_image* im, const g
         o.b25 = b25;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    if (st->precision == GM_PREC_FP16) launch_sym<__half>(iv, sv, eps, st->W, st->H, o, st->d, st->d32, s);
-    else if (st->precision == GM_PREC_BF16) launch_sym<__nv_bfloat16>(iv, sv, eps, st->W, st->H, o, st->d, st->d32, s);
-    else launch_sym<float>(iv, sv, eps, st->W, st->H, o, st->d, st->d32, s);
-    GM_CUDA_TRY(cudaGetLastError());
-    return GM_OK;
+    if (st->precision == GM_PREC_FP16) return launch_sym<__half>(iv, sv, eps, st->W, st->H, o, sms, s);
+    if (st->precision == GM_PREC_BF16) return launch_sym<__nv_bfloat16>(iv, sv, eps, st->W, st->H, o, sms, s);
+    return launch_sym<float>(iv, sv, eps, st->W, st->H, o, sms, s);
 }
 
 extern "C" int gm_levin_assemble_bands25(float* a, size_t apitch, float* b, const gm_image* im,
@@ -683,7 +923,8 @@ extern "C" int gm_levin_assemble_bands25(float* a, size_t apitch, float* b, cons
                                          void* stream)
 {
     if (!a || W <= 0 || H <= 0 || apitch < (size_t)W * H) { gm_set_error_msg("bad 25-band output"); return GM_ERR_INVALID; }
-    GM_TRY(gm_check_device(nullptr));
+    int sms = 0;
+    GM_TRY(gm_check_device(&sms));
     ImgView iv;
     ScribView sv;
     GM_TRY(make_views(im, sc, W, iv, sv));
@@ -692,15 +933,13 @@ extern "C" int gm_levin_assemble_bands25(float* a, size_t apitch, float* b, cons
     if (arithmetic == GM_ASSEMBLY_REFERENCE) {
         levin_ref_kernel<<<grid, TW * TH, 0, s>>>(iv, sv, (float)eps, W, H, a, apitch, b);
     } else {
-        // FP64 path through a scratch symmetric store.
-        gm_levin_store tmp;
-        GM_TRY(gm_levin_store_alloc(&tmp, W, H, GM_PREC_FP32));
-        BandedMatrix bm;
-        bm.a = a; bm.apitch = apitch; bm.bands = nullptr; bm.nbands = 25; bm.rows = W * H; bm.cols = W * H;
-        int rc = gm_levin_assemble(&tmp, im, sc, eps, &bm, b, stream);
-        cudaStreamSynchronize(s);
-        gm_levin_store_free(&tmp);
-        if (rc != GM_OK) return rc;
+        if (!(eps >= 0.0)) { gm_set_error_msg("eps must be >= 0"); return GM_ERR_INVALID; }
+        SymOut o;
+        memset(&o, 0, sizeof(o));
+        o.a25 = a;
+        o.apitch = apitch;
+        o.b25 = b;
+        return launch_sym<float>(iv, sv, eps, W, H, o, sms, s);
     }
     GM_CUDA_TRY(cudaGetLastError());
     return GM_OK;

@@ -116,3 +116,54 @@ def test_assembly_per_pixel_gamma_maps(orc):
     torch.cuda.synchronize()
     assert np.array_equal(st.planes("gamma")[:, :W].cpu().numpy(), gam)
     assert np.array_equal(st.planes("b")[:, :W].cpu().numpy(), gam * s)
+
+
+@pytest.mark.parametrize("W,H,prec,fmt", [(1, 9, "fp16", "rgb8"), (9, 2, "fp32", "rgba"), (3, 3, "bf16", "rgb8"),
+                                          (125, 5, "fp16", "rgba"), (126, 41, "fp16", "rgb8"), (127, 4, "fp32", "rgb8"),
+                                          (128, 3, "bf16", "rgba"), (253, 37, "fp32", "rgba"),
+                                          (1241, 130, "fp16", "rgb8")])
+def test_fp64_assembly_at_strip_and_run_edges(orc, W, H, prec, fmt):
+    """Widths around the kernel's 126-column strips, runs of 2 rows up to
+    several, images without a window.  Couplings within one FP32 ulp of the
+    oracle's plus what FP64 rounding allows either side: an error of 2^-53 in
+    81 Sigma (entries up to 81) over its smallest eigenvalue, at least 9 eps.
+    The diagonals are the FP64 sums of the stored weights, rounded once;
+    25-band output included."""
+    torch = torch_cuda()
+    from gpumatting_b200 import api
+
+    rng = np.random.default_rng(W * 1000 + H)
+    base = rng.integers(0, 256, size=(H // 4 + 2, W // 4 + 2, 3)).repeat(4, 0).repeat(4, 1)[:H, :W]
+    image = np.clip(base + rng.integers(-6, 7, size=(H, W, 3)), 0, 255).astype(np.uint8)
+    scr = rng.choice(np.array([0, 128, 255], np.uint8), size=(H, W), p=[0.1, 0.8, 0.1])
+    img = torch.from_numpy(image).cuda()
+    ref_in = image.astype(np.float64) / 255.0
+    if fmt == "rgba":
+        img = torch.from_numpy(np.concatenate([ref_in, np.ones((H, W, 1))], axis=2).astype(np.float32)).cuda()
+        ref_in = img.cpu().numpy()[..., :3].astype(np.float64)
+    w = orc.levin_sym64(np.ascontiguousarray(ref_in), 1e-5).reshape(12, H, W)
+    st = api.LevinStore(W, H, prec)
+    Lm = api.DeviceBandedMatrix(torch.zeros((25, W * H), device="cuda"), torch.tensor(orc.levin_offsets(W)).cuda(),
+                                W * H)
+    st.assemble(img, torch.from_numpy(scr).cuda(), eps=1e-5, gamma_value=100.0, bands25=Lm)
+    w32 = st.planes("w32")[:, :, :W].cpu().numpy()
+    sp = np.spacing(np.abs(w).astype(np.float32)).astype(np.float64)
+    assert np.all(np.abs(w32 - w) <= sp + 81 * 2.0 ** -53 / (9 * 1e-5))
+    wl = st.planes("w")[:, :, :W].float().cpu().numpy()
+    assert np.all(np.abs(wl - w) <= np.abs(w) * {"fp16": 2.0 ** -10, "bf16": 2.0 ** -7, "fp32": 2.0 ** -22}[prec] + 1e-7)
+    g = np.where(scr != 128, 100.0, 0.0)
+    for name, wp in (("d32", w32), ("d", wl)):
+        s = _row_diag(wp.astype(np.float64), g.ravel(), W, H)
+        got = st.planes(name)[:, :W].cpu().numpy().ravel()
+        assert np.all(np.abs(got - s) <= 0.5 * np.spacing(np.abs(s).astype(np.float32)) * (1 + 1e-6) + 1e-30), name
+    a = Lm.a.cpu().numpy().reshape(25, H, W)
+    for k in range(1, 13):
+        dv = (k + 2) // 5
+        du = k - 5 * dv
+        assert np.array_equal(a[12 + k], -w32[k - 1])
+        u0, u1 = max(0, du), min(W, W + du)
+        if u1 > u0 and H > dv:
+            assert np.array_equal(a[12 - k][dv:, u0:u1], -w32[k - 1][: H - dv, u0 - du:u1 - du])
+    a2, b2 = api.levin_bands25(img, torch.from_numpy(scr).cuda(), eps=1e-5, gamma_value=100.0, arithmetic="fp64")
+    assert np.array_equal(a2.cpu().numpy().view(np.uint32), Lm.a.cpu().numpy().view(np.uint32))
+    assert np.array_equal(b2.cpu().numpy().reshape(H, W), np.where(scr == 255, 100.0, 0.0).astype(np.float32))
