@@ -18,12 +18,13 @@
 //
 // V-cycle on level l with right-hand side b: x1 = omega b / D,
 // b_{l+1} = P^T (b - A x1), recurse, y = x1 + scale P x_{l+1},
-// x = y + omega (b - A y) / D.  Each level above the tail costs two streaming
+// x = y + omega (b - A y) / D.  Each level above the dense one costs two streaming
 // kernels ("down": smoothing + residual + restriction; "up": prolongation +
 // smoothing), both the persistent TMA-ring stencil kernel mg_fine_kernel; x1
-// is recomputed from b in "up" instead of stored.  The small levels at the
-// bottom (up to 160 KB of operators) run in one CTA (mg_tail_kernel), staged
-// in shared memory with block barriers between their phases.
+// is recomputed from b in "up" instead of stored.  From the first level of at
+// most kDenseMax cells down, the cycle is one dense matrix, formed once per
+// solve (mg_dense_build_kernel) and applied as a matrix-vector product
+// (mg_dense_kernel).
 //
 // Outer loop: PCG with FP64 solution (plus an FP32 increment folded in after
 // each replacement), FP32 vectors and FP64 scalars on the true FP32 operator;
@@ -102,12 +103,13 @@ struct Lev {
     float* gam;           // summed scribble weight (l >= 1)
     float* b;             // right-hand side of the V-cycle on this level
     float* x;             // V-cycle result on this level
+    double* M;            // levels lt .. L: the V-cycle from this level down as a dense matrix [n][n]
 };
 
 struct Args {
     Lev lev[kMaxLevels];
     int L;                // index of the coarsest level
-    int lt;               // first level of the single-CTA tail (1 <= lt <= L)
+    int lt;               // the level whose V-cycle is applied as a dense matrix (1 <= lt <= L)
     int W, H, P;          // fine grid (== lev[0])
     const float* w32;     // true operator: FP32 planes, gamma and d32 = gamma + row sum
     size_t ps32;
@@ -120,7 +122,6 @@ struct Args {
     double* x;            // FP64 solution [H][P]; the solution is x + xinc
     float* xinc;          // FP32 increment since the last replacement [H][P]
     float *r, *q, *p0, *p1;  // fine vectors [H][P]; z is lev[0].x
-    double* minv;         // coarsest inverse [n][n]
     double* parts;        // [5][kMaxParts]: pq, rr, true rr + bb, rz
     State* st;
     double rtol;
@@ -399,148 +400,148 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
 // V-cycle kernels
 // ---------------------------------------------------------------------------
 
-// The small levels lt .. L of a V-cycle in ONE CTA: their operators and
-// vectors are staged in shared memory (compact [H_l][W_l] arrays) and the
-// phases (smoothing + restriction down to the coarsest level, the exact
-// coarsest solve with the stored FP64 inverse, prolongation + smoothing back
-// up) are separated by block barriers instead of kernel launches.  Reads
-// b_lt, writes x_lt.
-constexpr int kTailThreads = 1024;
-constexpr int kTailSmem = 160 * 1024;
+// The V-cycle from level lt down is a linear map of at most kDenseMax cells, so
+// it is formed once per solve as a dense FP64 matrix and applied as one
+// matrix-vector product, spread over the GPU.  On level l, with S the
+// couplings, R = (1 - omega) I + omega D^-1 S and T = R P, the smoothing
+// steps and the coarse correction compose to
+//     M_l = omega D^-1 + R omega D^-1 + scale T M_{l+1} T^T,
+// from M_L, the coarsest inverse.  A row of T has four entries: a cell couples
+// to its own aggregate and to the three on its side of it.
+// Run level by level in one CTA these levels took 15-24 us of every
+// iteration (17 block barriers, and 75 KB staged by one SM); the product takes
+// 3-5, and forming the matrix 20-40 us per solve.  Per iteration: 46.0 -> 37.6
+// us at 317 x 211, 58.2 -> 47.2 at 640 x 480, 117.4 -> 106.5 at 1080p.
+struct TRow {
+    double w[4];  // own aggregate, x side, y side, diagonal
+    int I[4];
+};
 
-__device__ __forceinline__ float tail_sum(const float* c, const float* v, int W, int H, int n, int x, int y)
+__device__ __forceinline__ TRow t_row(const Lev& F, const Lev& C, int i, double om)
 {
-    const int i = y * W + x;
-    float s = 0.f;
+    const int x = i % F.W, y = i / F.W;
+    const float* c = static_cast<const float*>(F.c);
+    const size_t o = (size_t)y * F.P + x;
+    const int sx = (x & 1) ? 1 : -1, sy = (y & 1) ? 1 : -1;
+    const int X = x >> 1, Y = y >> 1;
+    double own = 0.0, wx = 0.0, wy = 0.0, wd = 0.0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int du = CoarseSten::du(k), dv = CoarseSten::dv(k);
-        const int xu = x + du, yu = y + dv, xl = x - du, yl = y - dv;
-        if (xu >= 0 && xu < W && yu < H) s = fmaf(c[k * n + i], v[yu * W + xu], s);
-        if (xl >= 0 && xl < W && yl >= 0) s = fmaf(c[k * n + yl * W + xl], v[yl * W + xl], s);
-    }
-    return s;
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            const int du = dir ? -CoarseSten::du(k) : CoarseSten::du(k), dv = dir ? -CoarseSten::dv(k) : CoarseSten::dv(k);
+            const int xj = x + du, yj = y + dv;
+            if (xj < 0 || xj >= F.W || yj < 0 || yj >= F.H) continue;
+            const double w = c[(size_t)k * F.ps + (dir ? (size_t)yj * F.P + xj : o)];
+            const bool ox = du == sx, oy = dv == sy;  // leaves the aggregate in x, in y
+            if (ox && oy) wd += w;
+            else if (ox) wx += w;
+            else if (oy) wy += w;
+            else own += w;
+        }
+    const double di = F.Di[o];
+    TRow t;
+    t.w[0] = di > 0.0 ? (1.0 - om) + om * di * own : 1.0;
+    t.w[1] = om * di * wx;
+    t.w[2] = om * di * wy;
+    t.w[3] = om * di * wd;
+    // a side outside the grid has no coupling; its index only has to be readable
+    const int Xs = min(max(X + sx, 0), C.W - 1), Ys = min(max(Y + sy, 0), C.H - 1);
+    t.I[0] = Y * C.W + X;
+    t.I[1] = Y * C.W + Xs;
+    t.I[2] = Ys * C.W + X;
+    t.I[3] = Ys * C.W + Xs;
+    return t;
 }
 
-__global__ void __launch_bounds__(kTailThreads) mg_tail_kernel(Args a)
+// Cells of the largest dense level.  Us per iteration with 700 / 1300 / 2100:
+// 42.1 / 37.6 / 39.2 at 317 x 211 (420 or 1080 cells), 50.7 / 47.2 / 52.6 at
+// 640 x 480 (300 or 1200), 103.8 / 106.5 / 111.1 at 1080p (510, 510, 2040): one
+// level less costs a row of 2 K doubles per warp, more than its two launches.
+constexpr int kDenseMax = 1300;
+constexpr int kDenseRows = 8;     // rows of M_l per CTA
+
+// Rows kDenseRows * blockIdx.x .. of M_l; thread j forms the entries of column j.
+__global__ void __launch_bounds__(kThreads) mg_dense_build_kernel(Args a, int l)
 {
-    // The levels' operators and the coarsest inverse were written by the
-    // set-up kernels, which completed before this kernel's predecessor
-    // started (every other kernel waits before it triggers), so they are
-    // staged before the wait, overlapping the predecessor; b_lt after it.
-    pdl_trigger();
-    extern __shared__ __align__(16) float sh[];
-    const int lt = a.lt, L = a.L, tid = threadIdx.x;
-    const float om = a.omega, sc = a.scale;
-    // carve: per level c[4n], 1/D [n], b[n], x[n]; then tmp[n_lt]; then the
-    // coarsest inverse (FP64, rounded up to an 8-byte boundary)
-    auto base = [&](int l) {
-        int off = 0;
-        for (int m = lt; m < l; ++m) off += 7 * a.lev[m].W * a.lev[m].H;
-        return sh + off;
-    };
-    float* tmp = base(L + 1);
-    const int nL = a.lev[L].W * a.lev[L].H;
-    double* minv = reinterpret_cast<double*>(sh + ((int)(tmp - sh) + a.lev[lt].W * a.lev[lt].H + 1) / 2 * 2);
-    for (int l = lt; l <= L; ++l) {
-        const Lev& G = a.lev[l];
-        const int W = G.W, n = G.W * G.H;
-        float* c = base(l);
-        float* D = c + 4 * n;
-        const float* gc = static_cast<const float*>(G.c);
-        for (int i = tid; i < n; i += kTailThreads) {
-            const size_t g = (size_t)(i / W) * G.P + i % W;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) c[k * n + i] = gc[(size_t)k * G.ps + g];
-            D[i] = G.Di[g];
+    pdl_enter();
+    __shared__ TRow rows[kDenseRows];
+    const Lev& F = a.lev[l];
+    const Lev& C = a.lev[l + 1];
+    const int n = F.W * F.H, nc = C.W * C.H;
+    const double om = (double)a.omega, sc = (double)a.scale;
+    const double* Mc = C.M;
+    const float* c = static_cast<const float*>(F.c);
+    for (int i0 = blockIdx.x * kDenseRows; i0 < n; i0 += gridDim.x * kDenseRows) {
+        if (threadIdx.x < kDenseRows && i0 + (int)threadIdx.x < n) rows[threadIdx.x] = t_row(F, C, i0 + threadIdx.x, om);
+        __syncthreads();
+        for (int j = threadIdx.x; j < n; j += kThreads) {
+            const TRow tj = t_row(F, C, j, om);
+            const int xj = j % F.W, yj = j / F.W;
+            const size_t oj = (size_t)yj * F.P + xj;
+            const double dj = F.Di[oj];
+            for (int q = 0; q < kDenseRows && i0 + q < n; ++q) {
+                const int i = i0 + q, xi = i % F.W, yi = i / F.W;
+                double v = 0.0;
+    #pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const double* row = Mc + (size_t)rows[q].I[e] * nc;
+                    v += rows[q].w[e] * (tj.w[0] * row[tj.I[0]] + tj.w[1] * row[tj.I[1]] + tj.w[2] * row[tj.I[2]] +
+                                         tj.w[3] * row[tj.I[3]]);
+                }
+                v *= sc;
+                const int du = xj - xi, dv = yj - yi;
+                if (i == j) v += om * (2.0 - om) * dj;
+                else if (du >= -1 && du <= 1 && dv >= -1 && dv <= 1) {
+                    // the coupling is stored at the upper end of the pair: planes E, SW, S, SE
+                    const bool up = dv > 0 || (dv == 0 && du > 0);
+                    const int k = dv == 0 ? 0 : 2 + (up ? du : -du);
+                    const size_t oi = (size_t)yi * F.P + xi;
+                    const double w = c[(size_t)k * F.ps + (up ? oi : oj)];
+                    v += om * om * w * (double)F.Di[oi] * dj;
+                }
+                F.M[(size_t)i * n + j] = v;
+            }
         }
+        __syncthreads();
     }
-    for (int i = tid; i < nL * nL; i += kTailThreads) minv[i] = a.minv[i];
+}
+
+// x_lt = M_lt b_lt, one warp per row.  The rows are constant during a solve
+// and were written before this kernel's predecessor started, so they are
+// loaded into registers ahead of the wait for b_lt.
+constexpr int kDenseLoads = (kDenseMax + 31) / 32;
+__global__ void __launch_bounds__(kThreads) mg_dense_kernel(Args a)
+{
+    pdl_trigger();
+    __shared__ float b[kDenseMax];
+    const Lev& G = a.lev[a.lt];
+    const int n = G.W * G.H, lane = threadIdx.x & 31, step = gridDim.x * (kThreads / 32);
+    int i = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    double m[kDenseLoads];
+    auto load_row = [&]() {
+        const double* row = G.M + (size_t)min(i, n - 1) * n;
+#pragma unroll
+        for (int q = 0; q < kDenseLoads; ++q) m[q] = lane + 32 * q < n ? __ldg(row + lane + 32 * q) : 0.0;
+    };
+    load_row();
     pdl_wait();
     if (a.st->done) return;
-    {
-        const Lev& G = a.lev[lt];
-        const int n = G.W * G.H;
-        float* b = base(lt) + 5 * n;
-        for (int i = tid; i < n; i += kTailThreads) b[i] = G.b[(size_t)(i / G.W) * G.P + i % G.W];
-    }
+    for (int j = threadIdx.x; j < n; j += kThreads) b[j] = G.b[(size_t)(j / G.W) * G.P + j % G.W];
     __syncthreads();
-    for (int l = lt; l < L; ++l) {
-        const Lev& F = a.lev[l];
-        const Lev& Cl = a.lev[l + 1];
-        const int W = F.W, H = F.H, n = W * H;
-        float* c = base(l);
-        float* D = c + 4 * n;
-        float* b = D + n;
-        float* x = b + n;
-        for (int i = tid; i < n; i += kTailThreads) x[i] = om * b[i] * D[i];
-        __syncthreads();
-        float* bc = base(l + 1) + 5 * Cl.W * Cl.H;
-        for (int I = tid; I < Cl.W * Cl.H; I += kTailThreads) {
-            const int X = I % Cl.W, Y = I / Cl.W;
-            float sum = 0.f;
-            for (int q = 0; q < 4; ++q) {
-                const int xf = 2 * X + (q & 1), yf = 2 * Y + (q >> 1);
-                if (xf < W && yf < H) {
-                    const int i = yf * W + xf;
-                    sum += rho_of(b[i], D[i], om, tail_sum(c, x, W, H, n, xf, yf));
-                }
-            }
-            bc[I] = sum;
-        }
-        __syncthreads();
+    for (;;) {
+        double s[2] = {0.0, 0.0};
+#pragma unroll
+        for (int q = 0; q < kDenseLoads; ++q)
+            if (lane + 32 * q < n) s[q & 1] = fma(m[q], (double)b[lane + 32 * q], s[q & 1]);
+        double t = s[0] + s[1];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0 && i < n) G.x[(size_t)(i / G.W) * G.P + i % G.W] = (float)t;
+        i += step;
+        if (i >= n) break;
+        load_row();
     }
-    {
-        const Lev& G = a.lev[L];
-        const int n = G.W * G.H;
-        float* b = base(L) + 5 * n;
-        float* x = b + n;
-        for (int i = tid; i < n; i += kTailThreads) {
-            double s = 0.0;
-#pragma unroll 8
-            for (int j = 0; j < n; ++j) s += minv[j * n + i] * (double)b[j];
-            x[i] = (float)s;
-        }
-        __syncthreads();
-    }
-    for (int l = L - 1; l >= lt; --l) {
-        const Lev& F = a.lev[l];
-        const Lev& Cl = a.lev[l + 1];
-        const int W = F.W, H = F.H, n = W * H;
-        float* c = base(l);
-        float* D = c + 4 * n;
-        float* b = D + n;
-        float* x = b + n;
-        const float* xc = base(l + 1) + 6 * Cl.W * Cl.H;
-        for (int i = tid; i < n; i += kTailThreads) {
-            const int xf = i % W, yf = i / W;
-            x[i] = fmaf(sc, xc[(yf >> 1) * Cl.W + (xf >> 1)], om * b[i] * D[i]);
-        }
-        __syncthreads();
-        for (int i = tid; i < n; i += kTailThreads) {
-            tmp[i] = smooth_of(x[i], b[i], D[i], om, tail_sum(c, x, W, H, n, i % W, i / W));
-        }
-        __syncthreads();
-        for (int i = tid; i < n; i += kTailThreads) x[i] = tmp[i];
-        __syncthreads();
-    }
-    {
-        const Lev& G = a.lev[lt];
-        const int n = G.W * G.H;
-        const float* x = base(lt) + 6 * n;
-        for (int i = tid; i < n; i += kTailThreads) G.x[(size_t)(i / G.W) * G.P + i % G.W] = x[i];
-    }
-}
-
-// Shared-memory bytes of the tail kernel for levels lt .. L.
-static int tail_bytes(const int* Wl, const int* Hl, int lt, int L)
-{
-    long long f = 0;
-    for (int l = lt; l <= L; ++l) f += 7LL * Wl[l] * Hl[l];
-    f += (long long)Wl[lt] * Hl[lt];
-    f = (f + 1) / 2 * 2;                        // the FP64 inverse starts 8-byte aligned
-    f += 2LL * Wl[L] * Hl[L] * Wl[L] * Hl[L];
-    return (int)(f * 4);
 }
 
 // ---------------------------------------------------------------------------
@@ -997,7 +998,7 @@ __global__ void __launch_bounds__(kThreads) mg_inverse_kernel(Args a)
         }
         return;
     }
-    for (int e = threadIdx.x; e < n * n; e += kThreads) a.minv[e] = A[e];
+    for (int e = threadIdx.x; e < n * n; e += kThreads) C.M[e] = A[e];
 }
 
 // 1 / d of the level-0 iteration diagonal (0 where d = 0).
@@ -1079,9 +1080,9 @@ static int make_plan(int W, int H, Plan& pl)
         if ((long long)w * h <= kCoarseMax) break;
     }
     pl.L = l;
-    // the tail takes the deepest levels that fit its shared memory
+    // the dense level: the first one small enough
     pl.lt = pl.L;
-    while (pl.lt > 1 && tail_bytes(pl.W, pl.H, pl.lt - 1, pl.L) <= kTailSmem) --pl.lt;
+    while (pl.lt > 1 && (long long)pl.W[pl.lt - 1] * pl.H[pl.lt - 1] <= kDenseMax) --pl.lt;
     return GM_OK;
 }
 
@@ -1118,16 +1119,17 @@ static size_t carve(const Plan& pl, int P0, char* base, Args* a)
         float* gam = (float*)take(n * 4);
         float* b = (float*)take(n * 4);
         float* xl = (float*)take(n * 4);
+        const size_t cells = (size_t)pl.W[l] * pl.H[l];
+        double* M = l >= pl.lt ? (double*)take(cells * cells * 8) : nullptr;
         if (a) {
             Lev& v = a->lev[l];
             v.W = pl.W[l]; v.H = pl.H[l]; v.P = P;
-            v.c = c; v.ps = n; v.D = D; v.Di = Di; v.gam = gam; v.b = b; v.x = xl;
+            v.c = c; v.ps = n; v.D = D; v.Di = Di; v.gam = gam; v.b = b; v.x = xl; v.M = M;
         }
     }
-    double* minv = (double*)take((size_t)kCoarseMax * kCoarseMax * 8);
     double* parts = (double*)take((size_t)5 * kMaxParts * 8);
     State* st = (State*)take(sizeof(State));
-    if (a) { a->minv = minv; a->parts = parts; a->st = st; }
+    if (a) { a->parts = parts; a->st = st; }
     return off;
 }
 
@@ -1235,7 +1237,7 @@ static int tiles_of(int W, int H, int ty) { return ((W + kTX - 1) / kTX) * ((H +
 // of the fine iteration planes.  A dry pass only computes the launch shapes
 // (it sets the kernels' shared-memory limits before any stream capture).
 // Tensor maps of the TMA-pipelined kernels: the level-0 SpMV, and the
-// restriction / prolongation of every level below the tail.
+// restriction / prolongation of every level above the dense one.
 struct FineMaps {
     TMaps spmv, down[kMaxLevels], up[kMaxLevels];
 };
@@ -1359,9 +1361,8 @@ struct Enq {
     void vcycle() const
     {
         for (int l = 0; l < a.lt; ++l) down(l);
-        int Wl[kMaxLevels], Hl[kMaxLevels];
-        for (int l = 0; l <= a.L; ++l) { Wl[l] = a.lev[l].W; Hl[l] = a.lev[l].H; }
-        go(mg_tail_kernel, 1, tail_bytes(Wl, Hl, a.lt, a.L), kTailThreads, a);
+        const int n = a.lev[a.lt].W * a.lev[a.lt].H;
+        go(mg_dense_kernel, (n + kThreads / 32 - 1) / (kThreads / 32), 0, kThreads, a);
         for (int l = a.lt - 1; l >= 0; --l) up(l);
     }
 
@@ -1384,6 +1385,8 @@ struct Enq {
         const int n = a.lev[a.L].W * a.lev[a.L].H;
         const int sm = (int)(sizeof(double) * ((size_t)n * n + 2 * kCoarseMax));
         go(mg_inverse_kernel, 1, sm, kThreads, a);
+        for (int l = a.L - 1; l >= a.lt; --l)
+            go(mg_dense_build_kernel, (a.lev[l].W * a.lev[l].H + kDenseRows - 1) / kDenseRows, 0, kThreads, a, l);
     }
 
     void setup() const

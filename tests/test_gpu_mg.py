@@ -66,6 +66,20 @@ def test_vcycle_matches_oracle(orc, prec):
     assert err <= 1e-4, err
 
 
+@pytest.mark.parametrize("W,H", [(16, 15), (17, 16), (23, 3), (72, 72), (73, 72), (145, 37), (80, 131), (300, 17)])
+def test_vcycle_dense_level_shapes(orc, W, H):
+    """Sizes around the dense level's limits: the coarsest level alone, levels of
+    just under and just over its cell limit, odd sides.  Tolerance: the parity
+    bar of the FP32 V-cycle (1e-4)."""
+    torch = torch_cuda()
+    st, p, w, g, b = _store(orc, W, H, "fp16", seed=4)
+    M, lv = _oracle_levels(st, g, "fp16")
+    r = np.random.default_rng(W + H).standard_normal((H, W)).astype(np.float32)
+    z, _, _ = st.mg_inspect(torch.from_numpy(r).cuda(), 0)
+    ref = M.vcycle(lv, r.astype(np.float64))
+    assert np.linalg.norm(z.double().cpu().numpy() - ref) <= 1e-4 * np.linalg.norm(ref)
+
+
 @pytest.mark.parametrize("prec", ["fp16", "bf16", "fp32"])
 def test_mg_solve_to_rtol(orc, prec):
     torch = torch_cuda()
