@@ -35,11 +35,13 @@
 // convergence (the same reliable-update rule as the fused CG).
 // All scalars stay on the device: every reduction ends in the last CTA to
 // finish (fixed summation order, so results are deterministic), and the whole
-// solve is ONE CUDA graph launch whose iteration loop is a device-side
-// conditional WHILE node -- no host round trip per iteration.  Kernels are
+// solve is ONE CUDA graph launch with two device-side conditional WHILE loops,
+// over the residual replacements and, inside, over the iterations between
+// them -- no host round trip per iteration.  Kernels are
 // chained with programmatic dependent launch.  gm_levin_solve_mg_many runs
 // many such solves on concurrent streams.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -129,7 +131,9 @@ struct Args {
     int outer_low;  // the level-0 SpMV streams the FP16 iteration planes, not w32
     int spare;      // keeps the struct free of padding (it is compared bytewise)
     float omega, scale;
-    unsigned long long cond;  // conditional-node handle (0 = host-driven loop)
+    // conditional-node handles (0 = host-driven loop): the loop over iterations
+    // up to the next residual replacement, and the loop over replacements
+    unsigned long long cond, cond_outer;
 };
 
 // ---------------------------------------------------------------------------
@@ -225,9 +229,13 @@ __device__ __forceinline__ bool last_cta_total(double (&v)[NV], double* parts, u
     return true;
 }
 
-__device__ __forceinline__ void set_cond(const Args& a, unsigned v)
+// Whether the kernels of an iteration have nothing to do: the solve is over, or
+// the residual replacement at the end of the unrolled loop body is due first.
+__device__ __forceinline__ bool paused(const State* st) { return st->done || st->need_replace; }
+
+__device__ __forceinline__ void set_loop(unsigned long long h, bool go)
 {
-    if (a.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, v);
+    if (h) cudaGraphSetConditional((cudaGraphConditionalHandle)h, go ? 1u : 0u);
 }
 
 // The smoother steps written with 1 / D only.  With S = sum_j w_ij v_j, so
@@ -255,7 +263,10 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
 {
     pdl_enter();
     State* st = a.st;
-    if (st->done) return;
+    if (paused(st)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) set_loop(a.cond, false);
+        return;
+    }
     const int W = a.W, H = a.H, P = a.P;
     const int it = st->iter;
     const double al = st->alpha;
@@ -302,8 +313,10 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
         st->iter = k;
         st->rr = v[0];
         const bool conv = a.rtol > 0.0 && v[0] <= a.rtol * a.rtol * st->bn2;
-        if (conv || (a.replace_every > 0 && k % a.replace_every == 0) || k >= a.max_iters || !isfinite(v[0]))
-            st->need_replace = 1;
+        const bool replace =
+            conv || (a.replace_every > 0 && k % a.replace_every == 0) || k >= a.max_iters || !isfinite(v[0]);
+        if (replace) st->need_replace = 1;
+        set_loop(a.cond, !replace);
     }
 }
 
@@ -313,7 +326,13 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
 {
     pdl_enter();
     State* st = a.st;
-    if (st->done || !st->need_replace) return;
+    if (st->done || !st->need_replace) {
+        if (st->done && blockIdx.x == 0 && threadIdx.x == 0) {
+            set_loop(a.cond, false);
+            set_loop(a.cond_outer, false);
+        }
+        return;
+    }
     extern __shared__ __align__(16) unsigned char smem[];
     float* pt = reinterpret_cast<float*>(smem);
     double* xt = reinterpret_cast<double*>(smem + sizeof(float) * FineSten::NP * (kTY + kHalo) * kPW);
@@ -393,6 +412,8 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
             st->done = 1;
             st->status = a.rtol > 0.0 ? GM_ERR_NOT_CONVERGED : GM_OK;
         }
+        set_loop(a.cond, !st->done);
+        set_loop(a.cond_outer, !st->done);
     }
 }
 
@@ -526,7 +547,7 @@ __global__ void __launch_bounds__(kThreads) mg_dense_kernel(Args a)
     };
     load_row();
     pdl_wait();
-    if (a.st->done) return;
+    if (paused(a.st)) return;
     for (int j = threadIdx.x; j < n; j += kThreads) b[j] = G.b[(size_t)(j / G.W) * G.P + j % G.W];
     __syncthreads();
     for (;;) {
@@ -560,7 +581,7 @@ __global__ void __launch_bounds__(kThreads) mg_dense_kernel(Args a)
 //   FM_DOWN  input x1 = omega b / d; rho = b - A x1, summed over 2 x 2 blocks
 //            into the level-1 right-hand side.
 //   FM_UP    input y = x1 + scale x_1[aggregate]; z = y + omega (b - A y) / d,
-//            sums r . z (the last CTA forms beta and the loop condition).
+//            sums r . z (the last CTA forms beta).
 // ---------------------------------------------------------------------------
 enum { FM_SPMV = 0, FM_DOWN = 1, FM_UP = 2 };
 constexpr int kFTW = 128;             // output columns per tile
@@ -689,8 +710,7 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
         }
     pdl_enter();
     State* st = a.st;
-    if (st->done) {
-        if (MODE == FM_UP && blockIdx.x == 0 && threadIdx.x == 0) set_cond(a, 0u);
+    if (paused(st)) {
         // complete the stages with no vectors and let the plane loads land
         if (tid == 0)
             for (int k = 0; k < npre; ++k) mbar_arrive_only(&full[k]);
@@ -869,8 +889,6 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
                 st->status = GM_ERR_BREAKDOWN;
                 st->done = 1;
             }
-            const bool go = !st->done && st->iter < a.max_iters + 1;
-            set_cond(a, go ? 1u : 0u);
         }
     }
 }
@@ -1147,7 +1165,7 @@ struct Graph {
 struct Dev {
     void* ws = nullptr;
     size_t ws_bytes = 0;
-    cudaStream_t cap = nullptr, cap2 = nullptr, run = nullptr;
+    cudaStream_t cap = nullptr, cap2 = nullptr, cap3 = nullptr, run = nullptr;
     State* host_state = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
     std::vector<Graph> graphs;
@@ -1184,6 +1202,7 @@ static int dev_setup(Dev& d, size_t bytes)
     if (!d.cap) {
         GM_CUDA_TRY(cudaStreamCreateWithFlags(&d.cap, cudaStreamNonBlocking));
         GM_CUDA_TRY(cudaStreamCreateWithFlags(&d.cap2, cudaStreamNonBlocking));
+        GM_CUDA_TRY(cudaStreamCreateWithFlags(&d.cap3, cudaStreamNonBlocking));
         GM_CUDA_TRY(cudaStreamCreateWithFlags(&d.run, cudaStreamNonBlocking));
         GM_CUDA_TRY(cudaMallocHost((void**)&d.host_state, sizeof(State)));
         GM_CUDA_TRY(cudaEventCreate(&d.e0));
@@ -1393,61 +1412,109 @@ struct Enq {
     {
         go(mg_init_kernel, pointwise_tiles(), 0, kThreads, a);
         build();
-        replace();
-        vcycle();
     }
 
+    // Preconditioner, matrix product, update: nothing while a replacement is due.
     void iteration() const
     {
+        vcycle();
         fine<FM_SPMV>(0);
         go(mg_update_kernel, pointwise_tiles(), 0, kThreads, a);
-        replace();
-        vcycle();
     }
 
     void finish() const { go(mg_final_kernel, pointwise_tiles(), 0, kThreads, a); }
 };
 
-// Captures set-up + WHILE(iteration) + finish into one graph.
+// Iterations per pass of the inner loop.  Going round a WHILE node costs 3-6 us
+// more than the next kernel of a chain, and an iteration that is skipped
+// because the replacement comes first about 12, so a pass is as long as
+// divides the distance between replacements well.  With the replacement check
+// out of the iteration and ten iterations a pass: 37.6 -> 34.8 us per iteration
+// at 317 x 211, 47.2 -> 44.6 at 640 x 480, 106.5 -> 99.6 at 1080p.
+static int unroll_for(const Args& a)
+{
+    const int period = std::max(1, std::min(a.max_iters, a.replace_every > 0 ? a.replace_every : a.max_iters));
+    int best = 1, best_cost = INT_MAX;
+    for (int u = 1; u <= 10; ++u) {
+        const int passes = (int)std::min<long long>(1000, ((long long)std::min(period, 1000) + u - 1) / u);
+        const int cost = 5 * passes + 12 * (passes * u - std::min(period, 1000));
+        if (cost < best_cost) { best_cost = cost; best = u; }
+    }
+    return best;
+}
+
+// Adds a WHILE node to the capture on stream s (condition 1 at its start),
+// with the handle *h or, where that is 0, a new one; returns its body.
+static cudaError_t add_while(cudaStream_t s, cudaGraphConditionalHandle* h, cudaGraph_t* body)
+{
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t ndeps = 0;
+    cudaError_t e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &ndeps);
+    if (e != cudaSuccess) return e;
+    if (*h == 0) e = cudaGraphConditionalHandleCreate(h, g, 1, cudaGraphCondAssignDefault);
+    if (e != cudaSuccess) return e;
+    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = *h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    e = cudaGraphAddNode(&node, g, deps, ndeps, &cp);
+    if (e != cudaSuccess) return e;
+    *body = cp.conditional.phGraph_out[0];
+    return cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies);
+}
+
+// Captures the whole solve into one graph:
+//   set-up; WHILE { replacement; WHILE { unrolled iterations } }; finish.
+// The replacement kernel keeps or ends both loops, the update kernel ends the
+// inner one when a replacement is due.
 template <class T>
 static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec)
 {
-    cudaGraph_t g = nullptr;
-    a.cond = 0;
+    cudaGraph_t g = nullptr, outer = nullptr, inner = nullptr;
+    a.cond = a.cond_outer = 0;
     {
         const Enq<T> dry{a, d.sms, d.cap, true, &fm};
         dry.setup();
+        dry.replace();
         dry.iteration();
         dry.finish();
     }
     GM_CUDA_TRY(cudaStreamBeginCapture(d.cap, cudaStreamCaptureModeThreadLocal));
     Enq<T>{a, d.sms, d.cap, false, &fm}.setup();
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    cudaError_t e = cudaStreamGetCaptureInfo(d.cap, &cs, nullptr, &cg, &deps, &ndeps);
-    cudaGraphConditionalHandle h = 0;
-    cudaGraphNode_t node = nullptr;
-    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, cg, 1, cudaGraphCondAssignDefault);
+    cudaGraphConditionalHandle ho = 0, hi = 0;
+    cudaError_t e = add_while(d.cap, &ho, &outer);
     if (e == cudaSuccess) {
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = h;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        e = cudaGraphAddNode(&node, cg, deps, ndeps, &cp);
-    }
-    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(d.cap, &node, 1, cudaStreamSetCaptureDependencies);
-    if (e == cudaSuccess) {
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        e = cudaStreamBeginCaptureToGraph(d.cap2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        // (the body's capture ends on every path: an unfinished one would
+        // leave the stream unusable)
+        e = cudaStreamBeginCaptureToGraph(d.cap2, outer, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             Args ab = a;
-            ab.cond = (unsigned long long)h;
-            Enq<T>{ab, d.sms, d.cap2, false, &fm}.iteration();
-            cudaGraph_t bg = body;
-            e = cudaStreamEndCapture(d.cap2, &bg);
+            ab.cond_outer = (unsigned long long)ho;
+            cudaStreamCaptureStatus cs;
+            cudaGraph_t og = nullptr;
+            // the inner handle is needed by the replacement kernel, which
+            // comes before the inner node
+            e = cudaStreamGetCaptureInfo(d.cap2, &cs, nullptr, &og, nullptr, nullptr);
+            if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hi, og, 1, cudaGraphCondAssignDefault);
+            ab.cond = (unsigned long long)hi;
+            if (e == cudaSuccess) Enq<T>{ab, d.sms, d.cap2, false, &fm}.replace();
+            if (e == cudaSuccess) e = add_while(d.cap2, &hi, &inner);
+            if (e == cudaSuccess) {
+                e = cudaStreamBeginCaptureToGraph(d.cap3, inner, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+                if (e == cudaSuccess) {
+                    const Enq<T> q{ab, d.sms, d.cap3, false, &fm};
+                    for (int k = unroll_for(a); k > 0; --k) q.iteration();
+                    cudaGraph_t x = nullptr;
+                    e = cudaStreamEndCapture(d.cap3, &x);
+                }
+            }
+            cudaGraph_t x = nullptr;
+            const cudaError_t e1 = cudaStreamEndCapture(d.cap2, &x);
+            if (e == cudaSuccess) e = e1;
         }
     }
     if (e == cudaSuccess) Enq<T>{a, d.sms, d.cap, false, &fm}.finish();
@@ -1537,11 +1604,14 @@ static int run(Dev& d, const Args& a0, const FineMaps& fm, int tcode, cudaStream
         }
     }
     // Host-driven loop: the same kernels, the done flag read every 4 iterations.
-    a.cond = 0;
+    // (every pass takes an iteration or a replacement, and a replacement is
+    // followed by an iteration or the end)
+    a.cond = a.cond_outer = 0;
     Enq<T> q{a, d.sms, st, false, &fm};
     GM_CUDA_TRY(cudaEventRecord(d.e0, st));
     q.setup();
-    for (int it = 0; it <= a.max_iters + 4; it += 4) {
+    for (int it = 0; it <= a.max_iters + 4; ++it) {
+        q.replace();
         for (int k = 0; k < 4; ++k) q.iteration();
         GM_CUDA_TRY(cudaMemcpyAsync(d.host_state, a.st, sizeof(State), cudaMemcpyDeviceToHost, st));
         GM_CUDA_TRY(cudaStreamSynchronize(st));
