@@ -33,8 +33,8 @@
 // would stall the recurrence).  The true residual b - A x in FP64 arithmetic
 // replaces the recurrence every `replace_every` iterations and decides
 // convergence (the same reliable-update rule as the fused CG).
-// All scalars stay on the device: every reduction ends in the last CTA to
-// finish (fixed summation order, so results are deterministic), and the whole
+// All scalars stay on the device: every reduction adds per-CTA partials in a
+// fixed order (so results are deterministic), in the kernel that needs it, and the whole
 // solve is ONE CUDA graph launch with two device-side conditional WHILE loops,
 // over the residual replacements and, inside, over the iterations between
 // them -- no host round trip per iteration.  Kernels are
@@ -85,14 +85,26 @@ struct CoarseSten {
 };
 
 // Device-resident solver state (scalars of the outer PCG).
+//
+// The sums r.z, p.q and r.r of an iteration are left as per-CTA partials by
+// the kernel that forms them and added up by every CTA of the kernel that
+// needs them, in index order (so all agree bit for bit), while its first
+// loads are in flight; a last-CTA sum costs 2.5-4 us at the end of each of the
+// three kernels instead.  A field is never written by a kernel whose other
+// CTAs may still read it: the matrix product of iteration k reads rz[(k - 1) & 1]
+// and writes rz[k & 1], the update reads iter and writes iter_next, the
+// restriction takes iter_next over into iter.
 struct State {
-    double rz, pq, alpha, beta, rr, bn2, rr_true;
-    int iter, done, status, need_replace, replacements;
-    int fold_at;  // iteration whose update folds the FP32 increment into x
-    int restart;  // the next search direction is z alone (beta = 0)
-    unsigned ticket[8];
+    double rz[2], rr, bn2, rr_true;
+    int iter, iter_next, done, status, need_replace, replacements;
+    int fold_at;     // iteration whose update folds the FP32 increment into x
+    int restart_at;  // iteration whose search direction is z alone (beta = 0)
+    unsigned ticket[2];
 };
-enum { T_PQ = 0, T_RR = 1, T_TRUE = 2, T_RZ = 3 };
+enum { T_RR = 0, T_TRUE = 1 };
+// Partial sums: p.q of the matrix product, r.r of the update, the true r.r and
+// b.b of the replacement, r.z of the level-0 prolongation.
+enum { S_PQ = 0, S_RR = 1, S_TRUE = 2, S_RZ = 4 };
 
 // One level's operator and vectors (l >= 1: FP32 planes of its own; level 0
 // points into the store and the fine work vectors).
@@ -124,12 +136,13 @@ struct Args {
     double* x;            // FP64 solution [H][P]; the solution is x + xinc
     float* xinc;          // FP32 increment since the last replacement [H][P]
     float *r, *q, *p0, *p1;  // fine vectors [H][P]; z is lev[0].x
-    double* parts;        // [5][kMaxParts]: pq, rr, true rr + bb, rz
+    double* parts;        // [5][kMaxParts], S_*
+    int n_pq, n_rr, n_rz, spare0; // partials per sum: the CTAs of the kernel that leaves them
     State* st;
     double rtol;
     int max_iters, replace_every;
     int outer_low;  // the level-0 SpMV streams the FP16 iteration planes, not w32
-    int spare;      // keeps the struct free of padding (it is compared bytewise)
+    int spare;
     float omega, scale;
     // conditional-node handles (0 = host-driven loop): the loop over iterations
     // up to the next residual replacement, and the loop over replacements
@@ -229,6 +242,23 @@ __device__ __forceinline__ bool last_cta_total(double (&v)[NV], double* parts, u
     return true;
 }
 
+// This CTA's share of sum `which`, for the consuming kernel.
+__device__ __forceinline__ void publish(double v, const Args& a, int which)
+{
+    __shared__ double red[32];
+    double t[1] = {v};
+    block_sum<1>(t, red);
+    if (threadIdx.x == 0) a.parts[(size_t)which * kMaxParts + blockIdx.x] = t[0];
+}
+
+// The iteration now complete (k of them) ends the recurrence: converged by its
+// own residual, at the replacement period or at the limit.
+__device__ __forceinline__ bool replacement_due(const Args& a, const State* st, int k, double rr)
+{
+    return (a.rtol > 0.0 && rr <= a.rtol * a.rtol * st->bn2) || (a.replace_every > 0 && k % a.replace_every == 0) ||
+           k >= a.max_iters || !isfinite(rr);
+}
+
 // Whether the kernels of an iteration have nothing to do: the solve is over, or
 // the residual replacement at the end of the unrolled loop body is due first.
 __device__ __forceinline__ bool paused(const State* st) { return st->done || st->need_replace; }
@@ -255,34 +285,51 @@ __device__ __forceinline__ float smooth_of(float y, float b, float di, float om,
 // Outer PCG kernels (level 0)
 // ---------------------------------------------------------------------------
 
-// x += alpha p_new, r -= alpha q, partial r . r; the last CTA counts the
-// iteration and asks for a true-residual replacement when it is due.  Four
-// pixels per step (16-byte vectors; the pitch is a multiple of 8); lanes past
-// W are written as zero and left out of the sum.
+// x += alpha p_new, r -= alpha q, r . r, with alpha = r.z / p.q from the matrix
+// product's partials.  The last update of a loop pass (LAST) sums r . r itself
+// and decides whether the loop goes on; after the others the restriction does.
+// Four pixels per step (16-byte vectors; the pitch is a multiple of 8); lanes
+// past W are written as zero and left out of the sum.
+template <bool LAST>
 __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
 {
     pdl_enter();
     State* st = a.st;
-    if (paused(st)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) set_loop(a.cond, false);
-        return;
-    }
     const int W = a.W, H = a.H, P = a.P;
     const int it = st->iter;
-    const double al = st->alpha;
-    const float alf = (float)al;
+    const double rz = st->rz[it & 1];
     const float* pn = (it & 1) ? a.p0 : a.p1;
     const bool fold = st->fold_at == it;  // a replacement ran: move the increment into x
-    double acc = 0.0;
     const int qpr = (W + 3) / 4;
     const size_t nq = (size_t)qpr * H;
-    for (size_t qi = (size_t)blockIdx.x * kThreads + threadIdx.x; qi < nq; qi += (size_t)gridDim.x * kThreads) {
-        const int y = (int)(qi / qpr), x = (int)(qi % qpr) * 4;
-        const size_t o = (size_t)y * P + x;
-        const float4 p = *reinterpret_cast<const float4*>(pn + o);
-        const float4 q = *reinterpret_cast<const float4*>(a.q + o);
-        float4 r = *reinterpret_cast<const float4*>(a.r + o);
-        float4 xi = *reinterpret_cast<const float4*>(a.xinc + o);
+    size_t qi = (size_t)blockIdx.x * kThreads + threadIdx.x;
+    float4 p, q, r, xi;
+    size_t o = 0;
+    auto load = [&]() {
+        o = (qi / qpr) * P + (qi % qpr) * 4;
+        p = *reinterpret_cast<const float4*>(pn + o);
+        q = *reinterpret_cast<const float4*>(a.q + o);
+        r = *reinterpret_cast<const float4*>(a.r + o);
+        xi = *reinterpret_cast<const float4*>(a.xinc + o);
+    };
+    if (qi < nq) load();
+    const double pq = warp_sum_range(a.parts + (size_t)S_PQ * kMaxParts, 0, a.n_pq);
+    const bool stop = paused(st);  // (done is set below only when every thread returns)
+    const bool bad = !(pq > 0.0) || !isfinite(pq) || !isfinite(rz);
+    if (stop || bad) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (!stop) {
+                st->status = GM_ERR_BREAKDOWN;
+                st->done = 1;
+            }
+            if (LAST) set_loop(a.cond, false);
+        }
+        return;
+    }
+    const float alf = (float)(rz / pq);
+    double acc = 0.0;
+    for (; qi < nq; ) {
+        const int x = (int)(qi % qpr) * 4;
         const bool v1 = x + 1 < W, v2 = x + 2 < W, v3 = x + 3 < W;
         if (fold) {
             double2 x01 = *reinterpret_cast<const double2*>(a.x + o);
@@ -306,17 +353,21 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
         *reinterpret_cast<float4*>(a.xinc + o) = xi;
         *reinterpret_cast<float4*>(a.r + o) = r;
         acc += (double)r.x * r.x + (double)r.y * r.y + ((double)r.z * r.z + (double)r.w * r.w);
+        qi += (size_t)gridDim.x * kThreads;
+        if (qi < nq) load();
     }
-    double v[1] = {acc};
-    if (last_cta_total<1>(v, a.parts + kMaxParts, &st->ticket[T_RR]) && threadIdx.x == 0) {
-        const int k = it + 1;
-        st->iter = k;
-        st->rr = v[0];
-        const bool conv = a.rtol > 0.0 && v[0] <= a.rtol * a.rtol * st->bn2;
-        const bool replace =
-            conv || (a.replace_every > 0 && k % a.replace_every == 0) || k >= a.max_iters || !isfinite(v[0]);
-        if (replace) st->need_replace = 1;
-        set_loop(a.cond, !replace);
+    if (LAST) {
+        double v[1] = {acc};
+        if (last_cta_total<1>(v, a.parts + (size_t)S_RR * kMaxParts, &st->ticket[T_RR]) && threadIdx.x == 0) {
+            const bool replace = replacement_due(a, st, it + 1, v[0]);
+            st->iter = it + 1;
+            st->rr = v[0];
+            if (replace) st->need_replace = 1;
+            set_loop(a.cond, !replace);
+        }
+    } else {
+        publish(acc, a, S_RR);
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->iter_next = it + 1;
     }
 }
 
@@ -383,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
         }
     }
     double v[2] = {rr, bb};
-    if (last_cta_total<2>(v, a.parts + 2 * kMaxParts, &st->ticket[T_TRUE]) && threadIdx.x == 0) {
+    if (last_cta_total<2>(v, a.parts + (size_t)S_TRUE * kMaxParts, &st->ticket[T_TRUE]) && threadIdx.x == 0) {
         if (st->replacements == 0) st->bn2 = v[1];
         st->replacements += 1;
         st->fold_at = st->iter;
@@ -395,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
         // exists, and beta = true r.z / recurrence r.z would let it swamp
         // the new one (the iteration stalls), so the next direction restarts
         // from z.  Forward solves never open such a gap.
-        st->restart = v[0] > 4.0 * st->rr;
+        st->restart_at = v[0] > 4.0 * st->rr ? st->iter : -1;
         st->rr_true = v[0];
         st->rr = v[0];
         const double bn2 = st->bn2;
@@ -575,13 +626,15 @@ __global__ void __launch_bounds__(kThreads) mg_dense_kernel(Args a)
 // the image.  After a stage lands, the CTA forms the stencil input in a
 // shared tile, then each thread marches TH / 4 rows of a column pair with a
 // 5 x 6 window of it in registers.
-//   FM_SPMV  input z + beta p_old; q = A p_new with the FP32 planes and d32
-//            (FP16 planes and d when Args::outer_low);
-//            writes p_new and q, sums p_new . q (the last CTA forms alpha).
+//   FM_SPMV  input z + beta p_old, beta from the prolongation's r . z;
+//            q = A p_new with the FP32 planes and d32 (FP16 planes and d when
+//            Args::outer_low); writes p_new and q, sums p_new . q.
 //   FM_DOWN  input x1 = omega b / d; rho = b - A x1, summed over 2 x 2 blocks
-//            into the level-1 right-hand side.
+//            into the level-1 right-hand side.  On level 0 with `pending`: the
+//            update before it left r . r as partials, so this kernel counts
+//            the iteration and stops when a replacement is due.
 //   FM_UP    input y = x1 + scale x_1[aggregate]; z = y + omega (b - A y) / d,
-//            sums r . z (the last CTA forms beta).
+//            sums r . z.
 // ---------------------------------------------------------------------------
 enum { FM_SPMV = 0, FM_DOWN = 1, FM_UP = 2 };
 constexpr int kFTW = 128;             // output columns per tile
@@ -670,7 +723,7 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar, uint32_t parity, State
 
 template <int MODE, class S, class T>
 __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::NP>::THR, 1)
-    mg_fine_kernel(const __grid_constant__ TMaps tm, Args a, int l)
+    mg_fine_kernel(const __grid_constant__ TMaps tm, Args a, int l, int pending)
 {
     constexpr int ES = FinePlanes<MODE, T>::ES;
     using PT = typename FinePlanes<MODE, T>::PT;
@@ -710,16 +763,15 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
         }
     pdl_enter();
     State* st = a.st;
-    if (paused(st)) {
-        // complete the stages with no vectors and let the plane loads land
-        if (tid == 0)
-            for (int k = 0; k < npre; ++k) mbar_arrive_only(&full[k]);
-        for (int k = 0; k < npre; ++k) stage_wait(&full[k], 0u, st);
-        return;
-    }
+    // One thread looks: the lead CTA of this kernel may set need_replace or done
+    // while others start, and a CTA has to take one path.
+    __shared__ int s_stop;
+    if (tid == 0) s_stop = paused(st);
+    __syncthreads();
+    const bool stop = s_stop != 0;
     const int it = st->iter;
     const bool first = it == 0;
-    const float beta = (float)st->beta, om = a.omega, sc = a.scale;
+    const float om = a.omega, sc = a.scale;
     const CUtensorMap* mv1 = MODE == FM_SPMV ? ((it & 1) ? &tm.m[3] : &tm.m[2]) : &tm.m[2];
     float* pnew = (it & 1) ? a.p0 : a.p1;
     const Lev& C = a.lev[l + 1];
@@ -736,11 +788,57 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
         issue_planes(t, s);
         issue_vectors(t, s);
     };
+    auto drain = [&]() {  // complete the requested stages
+        for (int k = 0; k < npre; ++k) stage_wait(&full[k], 0u, st);
+    };
+    if (stop) {
+        if (tid == 0)
+            for (int k = 0; k < npre; ++k) mbar_arrive_only(&full[k]);
+        drain();
+        return;
+    }
     if (tid == 0)
         for (int k = 0; k < npre; ++k) {
             mbar_arrive_expect_tx(&full[k], LY::bytes - (uint32_t)LY::PB);
             issue_vectors(t0 + k * G, k);
         }
+    // Sums of the kernels before, added up while the vectors are on their way.
+    float beta = 0.f;
+    if (MODE == FM_SPMV || (MODE == FM_DOWN && pending)) {
+        __shared__ double s_sum;
+        if (tid >= 32 && tid < 64) {
+            const double t = MODE == FM_SPMV ? warp_sum_range(a.parts + (size_t)S_RZ * kMaxParts, 0, a.n_rz)
+                                             : warp_sum_range(a.parts + (size_t)S_RR * kMaxParts, 0, a.n_rr);
+            if (tid == 32) s_sum = t;
+        }
+        __syncthreads();
+        const double sum = s_sum;
+        const bool lead = blockIdx.x == 0 && tid == 0;
+        if (MODE == FM_SPMV) {
+            if (!isfinite(sum)) {
+                if (lead) {
+                    st->status = GM_ERR_BREAKDOWN;
+                    st->done = 1;
+                }
+                drain();
+                return;
+            }
+            if (!first && st->restart_at != it) beta = (float)(sum / st->rz[(it & 1) ^ 1]);
+            if (lead) st->rz[it & 1] = sum;
+        } else {
+            const int k = st->iter_next;
+            const bool replace = replacement_due(a, st, k, sum);
+            if (lead) {
+                st->iter = k;
+                st->rr = sum;
+                if (replace) st->need_replace = 1;
+            }
+            if (replace) {
+                drain();
+                return;
+            }
+        }
+    }
     const int cp = tid & 63, rg = tid >> 6;
     const int lu = 8 + 2 * cp;
     const int r0 = rg * RPT;
@@ -867,30 +965,8 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
     }
     if (!ok) return;
     static_assert(NT <= 1024, "");
-    if (MODE == FM_SPMV) {
-        double v[1] = {acc};
-        if (last_cta_total<1>(v, a.parts, &st->ticket[T_PQ]) && threadIdx.x == 0) {
-            st->pq = v[0];
-            if (!(v[0] > 0.0) || !isfinite(v[0]) || !isfinite(st->rz)) {
-                st->status = GM_ERR_BREAKDOWN;
-                st->done = 1;
-            } else {
-                st->alpha = st->rz / v[0];
-            }
-        }
-    } else if (MODE == FM_UP && l == 0) {
-        double v[1] = {acc};
-        if (last_cta_total<1>(v, a.parts + 4 * kMaxParts, &st->ticket[T_RZ]) && threadIdx.x == 0) {
-            const double rz = v[0];
-            if (st->iter > 0) st->beta = st->restart ? 0.0 : rz / st->rz;
-            st->restart = 0;
-            st->rz = rz;
-            if (!isfinite(rz)) {
-                st->status = GM_ERR_BREAKDOWN;
-                st->done = 1;
-            }
-        }
-    }
+    if (MODE == FM_SPMV) publish(acc, a, S_PQ);
+    else if (MODE == FM_UP && l == 0) publish(acc, a, S_RZ);
 }
 
 // ---------------------------------------------------------------------------
@@ -1045,15 +1121,16 @@ __global__ void mg_init_kernel(Args a)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         State* st = a.st;
-        st->rz = st->pq = st->alpha = st->beta = st->rr = st->bn2 = st->rr_true = 0.0;
+        st->rz[0] = st->rz[1] = st->rr = st->bn2 = st->rr_true = 0.0;
         st->iter = 0;
+        st->iter_next = 0;
         st->done = 0;
         st->status = GM_OK;
         st->need_replace = 1;
         st->replacements = 0;
         st->fold_at = -1;
-        st->restart = 0;
-        for (int k = 0; k < 8; ++k) st->ticket[k] = 0u;
+        st->restart_at = -1;
+        for (int k = 0; k < 2; ++k) st->ticket[k] = 0u;
     }
 }
 
@@ -1330,10 +1407,15 @@ struct Enq {
     bool dry;
     const FineMaps* fm;
 
+    template <class K> int ctas(K fn, int tiles, int smem, int threads) const
+    {
+        const int g = std::min(tiles, sms * occupancy((const void*)fn, smem, threads));
+        return std::max(1, std::min(g, kMaxParts));
+    }
+
     template <class K, class... X> void go(K fn, int tiles, int smem, int threads, X... args) const
     {
-        int g = std::min(tiles, sms * occupancy((const void*)fn, smem, threads));
-        g = std::max(1, std::min(g, kMaxParts));
+        const int g = ctas(fn, tiles, smem, threads);
         if (dry) return;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)g);
@@ -1355,34 +1437,44 @@ struct Enq {
 
     // The TMA-pipelined kernels: level 0 with the store's 12 planes in the
     // iteration precision, the levels below with their 4 FP32 planes.
-    template <int MODE> void fine(int l) const
+    template <int MODE> void fine(int l, int pending = 0) const
     {
-        const Lev& F = a.lev[l];
         const TMaps& m = MODE == FM_SPMV ? fm->spmv : (MODE == FM_DOWN ? fm->down[l] : fm->up[l]);
-        if (l == 0 && MODE == FM_SPMV && !a.outer_low) {
-            using LY = FineLayout<MODE, 4, 12>;
-            const int tiles = ((F.W + kFTW - 1) / kFTW) * ((F.H + LY::TH - 1) / LY::TH);
-            go(mg_fine_kernel<MODE, FineSten, float>, tiles, LY::total, LY::THR, m, a, 0);
-        } else if (l == 0) {
-            using LY = FineLayout<MODE, FinePlanes<MODE, T>::ES, 12>;
-            const int tiles = ((F.W + kFTW - 1) / kFTW) * ((F.H + LY::TH - 1) / LY::TH);
-            go(mg_fine_kernel<MODE, FineSten, T>, tiles, LY::total, LY::THR, m, a, 0);
-        } else {
-            using LY = FineLayout<MODE, 4, 4>;
-            const int tiles = ((F.W + kFTW - 1) / kFTW) * ((F.H + LY::TH - 1) / LY::TH);
-            go(mg_fine_kernel<MODE, CoarseSten, float>, tiles, LY::total, LY::THR, m, a, l);
-        }
+        with_fine<MODE>(l, [&](auto fn, int tiles, int smem, int threads) { go(fn, tiles, smem, threads, m, a, l, pending); });
     }
 
-    void down(int l) const { fine<FM_DOWN>(l); }
-    void up(int l) const { fine<FM_UP>(l); }
-
-    void vcycle() const
+    // The kernel and launch shape of one level's pass.
+    template <int MODE, class F> auto with_fine(int l, F f) const
     {
-        for (int l = 0; l < a.lt; ++l) down(l);
+        const Lev& G = a.lev[l];
+        auto tiles = [&](int th) { return ((G.W + kFTW - 1) / kFTW) * ((G.H + th - 1) / th); };
+        if (l > 0) {
+            using LY = FineLayout<MODE, 4, 4>;
+            return f(mg_fine_kernel<MODE, CoarseSten, float>, tiles(LY::TH), LY::total, LY::THR);
+        }
+        if (MODE == FM_SPMV && !a.outer_low) {
+            using LY = FineLayout<MODE, 4, 12>;
+            return f(mg_fine_kernel<MODE, FineSten, float>, tiles(LY::TH), LY::total, LY::THR);
+        }
+        using LY = FineLayout<MODE, FinePlanes<MODE, T>::ES, 12>;
+        return f(mg_fine_kernel<MODE, FineSten, T>, tiles(LY::TH), LY::total, LY::THR);
+    }
+
+    // Partials per sum: the CTAs of the kernels that leave them.
+    void count_parts(Args& out) const
+    {
+        auto n = [&](auto fn, int tiles, int smem, int threads) { return ctas(fn, tiles, smem, threads); };
+        out.n_pq = with_fine<FM_SPMV>(0, n);
+        out.n_rz = with_fine<FM_UP>(0, n);
+        out.n_rr = ctas(mg_update_kernel<false>, pointwise_tiles(), 0, kThreads);
+    }
+
+    void vcycle(int pending) const
+    {
+        for (int l = 0; l < a.lt; ++l) fine<FM_DOWN>(l, l == 0 ? pending : 0);
         const int n = a.lev[a.lt].W * a.lev[a.lt].H;
         go(mg_dense_kernel, (n + kThreads / 32 - 1) / (kThreads / 32), 0, kThreads, a);
-        for (int l = a.lt - 1; l >= 0; --l) up(l);
+        for (int l = a.lt - 1; l >= 0; --l) fine<FM_UP>(l);
     }
 
     void replace() const
@@ -1414,12 +1506,16 @@ struct Enq {
         build();
     }
 
-    // Preconditioner, matrix product, update: nothing while a replacement is due.
-    void iteration() const
+    // One loop pass of preconditioner, matrix product and update; an iteration
+    // does nothing when a replacement is due before it.
+    void iterations(int count) const
     {
-        vcycle();
-        fine<FM_SPMV>(0);
-        go(mg_update_kernel, pointwise_tiles(), 0, kThreads, a);
+        for (int k = 0; k < count; ++k) {
+            vcycle(k > 0);
+            fine<FM_SPMV>(0);
+            if (k + 1 < count) go(mg_update_kernel<false>, pointwise_tiles(), 0, kThreads, a);
+            else go(mg_update_kernel<true>, pointwise_tiles(), 0, kThreads, a);
+        }
     }
 
     void finish() const { go(mg_final_kernel, pointwise_tiles(), 0, kThreads, a); }
@@ -1477,10 +1573,11 @@ static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec
     cudaGraph_t g = nullptr, outer = nullptr, inner = nullptr;
     a.cond = a.cond_outer = 0;
     {
-        const Enq<T> dry{a, d.sms, d.cap, true, &fm};
+        const Enq<T> dry{a, d.sms, d.cap, true, &fm};  // sets the kernels' shared-memory limits too
         dry.setup();
         dry.replace();
-        dry.iteration();
+        dry.iterations(2);
+        dry.count_parts(a);
         dry.finish();
     }
     GM_CUDA_TRY(cudaStreamBeginCapture(d.cap, cudaStreamCaptureModeThreadLocal));
@@ -1507,7 +1604,7 @@ static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec
                 e = cudaStreamBeginCaptureToGraph(d.cap3, inner, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
                 if (e == cudaSuccess) {
                     const Enq<T> q{ab, d.sms, d.cap3, false, &fm};
-                    for (int k = unroll_for(a); k > 0; --k) q.iteration();
+                    q.iterations(unroll_for(a));
                     cudaGraph_t x = nullptr;
                     e = cudaStreamEndCapture(d.cap3, &x);
                 }
@@ -1607,12 +1704,13 @@ static int run(Dev& d, const Args& a0, const FineMaps& fm, int tcode, cudaStream
     // (every pass takes an iteration or a replacement, and a replacement is
     // followed by an iteration or the end)
     a.cond = a.cond_outer = 0;
+    Enq<T>{a, d.sms, st, true, &fm}.count_parts(a);
     Enq<T> q{a, d.sms, st, false, &fm};
     GM_CUDA_TRY(cudaEventRecord(d.e0, st));
     q.setup();
     for (int it = 0; it <= a.max_iters + 4; ++it) {
         q.replace();
-        for (int k = 0; k < 4; ++k) q.iteration();
+        q.iterations(4);
         GM_CUDA_TRY(cudaMemcpyAsync(d.host_state, a.st, sizeof(State), cudaMemcpyDeviceToHost, st));
         GM_CUDA_TRY(cudaStreamSynchronize(st));
         if (d.host_state->done) break;
@@ -1973,7 +2071,7 @@ extern "C" int gm_levin_mg_inspect(const gm_levin_store* store, int use_low, con
         if (r && z) {
             cudaMemcpy2DAsync(a.r, (size_t)a.P * 4, r, (size_t)a.W * 4, (size_t)a.W * 4, a.H, cudaMemcpyDeviceToDevice,
                               st);
-            q.vcycle();
+            q.vcycle(0);
             cudaMemcpy2DAsync(z, (size_t)a.W * 4, a.lev[0].x, (size_t)a.P * 4, (size_t)a.W * 4, a.H,
                               cudaMemcpyDeviceToDevice, st);
         }

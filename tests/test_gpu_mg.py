@@ -361,6 +361,25 @@ def test_mg_host_loop_matches_graph(orc, tmp_path):
     assert np.array_equal(outs["0"][1].view(np.uint32), outs["1"][1].view(np.uint32))
 
 
+@pytest.mark.parametrize("every,count", [(50, 1), (50, 2), (50, 11), (50, 60), (1, 4), (3, 10), (7, 30), (11, 30), (0, 23)])
+def test_mg_replacement_periods(orc, monkeypatch, every, count):
+    """Fixed counts with replacement periods that do and do not divide the loop
+    pass: the iterations and replacements asked for, exactly, and the same
+    bits as the host-driven loop (which has other passes)."""
+    torch = torch_cuda()
+    W, H = 150, 70
+    st, p, w, g, b = _store(orc, W, H, "fp16")
+    outs = []
+    for mode in ("1", "0"):
+        monkeypatch.setenv("GM_MG_GRAPH", mode)
+        alpha = torch.full((H, W), 0.5, device="cuda")
+        res = st.solve(alpha, "mg", rtol=0.0, max_iters=count, replace_every=every)
+        due = sum(1 for k in range(1, count + 1) if k == count or (every > 0 and k % every == 0))
+        assert res.status == 0 and res.iters == count and res.replacements == 1 + due
+        outs.append(alpha.cpu().numpy())
+    assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32))
+
+
 def test_batch_solve_with_mg(orc):
     """gm_batch_solve with GM_SOLVER_MG gives every image of the canvas its own
     one-graph MG solve (concurrent streams): each result matches, bit for bit
