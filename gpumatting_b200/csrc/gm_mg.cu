@@ -293,26 +293,36 @@ __device__ __forceinline__ float smooth_of(float y, float b, float di, float om,
 template <bool LAST>
 __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
 {
-    pdl_enter();
+    // What kernels before the predecessor left (they are complete: the
+    // predecessor started after them) is read ahead of the wait for it.
     State* st = a.st;
     const int W = a.W, H = a.H, P = a.P;
     const int it = st->iter;
-    const double rz = st->rz[it & 1];
-    const float* pn = (it & 1) ? a.p0 : a.p1;
     const bool fold = st->fold_at == it;  // a replacement ran: move the increment into x
+    const float* pn = (it & 1) ? a.p0 : a.p1;
     const int qpr = (W + 3) / 4;
-    const size_t nq = (size_t)qpr * H;
-    size_t qi = (size_t)blockIdx.x * kThreads + threadIdx.x;
-    float4 p, q, r, xi;
-    size_t o = 0;
-    auto load = [&]() {
-        o = (qi / qpr) * P + (qi % qpr) * 4;
-        p = *reinterpret_cast<const float4*>(pn + o);
-        q = *reinterpret_cast<const float4*>(a.q + o);
-        r = *reinterpret_cast<const float4*>(a.r + o);
-        xi = *reinterpret_cast<const float4*>(a.xinc + o);
+    const size_t nq = (size_t)qpr * H, step = (size_t)gridDim.x * kThreads;
+    struct Quad {
+        size_t o;
+        int x;
+        float4 p, q, r, xi;
     };
-    if (qi < nq) load();
+    auto load_old = [&](Quad& d, size_t qi) {
+        d.x = (int)(qi % qpr) * 4;
+        d.o = (qi / qpr) * P + d.x;
+        d.r = *reinterpret_cast<const float4*>(a.r + d.o);
+        d.xi = *reinterpret_cast<const float4*>(a.xinc + d.o);
+    };
+    auto load_new = [&](Quad& d) {
+        d.p = *reinterpret_cast<const float4*>(pn + d.o);
+        d.q = *reinterpret_cast<const float4*>(a.q + d.o);
+    };
+    size_t qi = (size_t)blockIdx.x * kThreads + threadIdx.x;
+    Quad c, n;
+    if (qi < nq) load_old(c, qi);
+    pdl_enter();
+    if (qi < nq) load_new(c);
+    const double rz = st->rz[it & 1];
     const double pq = warp_sum_range(a.parts + (size_t)S_PQ * kMaxParts, 0, a.n_pq);
     const bool stop = paused(st);  // (done is set below only when every thread returns)
     const bool bad = !(pq > 0.0) || !isfinite(pq) || !isfinite(rz);
@@ -328,33 +338,35 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
     }
     const float alf = (float)(rz / pq);
     double acc = 0.0;
-    for (; qi < nq; ) {
-        const int x = (int)(qi % qpr) * 4;
-        const bool v1 = x + 1 < W, v2 = x + 2 < W, v3 = x + 3 < W;
-        if (fold) {
-            double2 x01 = *reinterpret_cast<const double2*>(a.x + o);
-            double2 x23 = *reinterpret_cast<const double2*>(a.x + o + 2);
-            x01.x += (double)xi.x;
-            x01.y = v1 ? x01.y + (double)xi.y : 0.0;
-            x23.x = v2 ? x23.x + (double)xi.z : 0.0;
-            x23.y = v3 ? x23.y + (double)xi.w : 0.0;
-            *reinterpret_cast<double2*>(a.x + o) = x01;
-            *reinterpret_cast<double2*>(a.x + o + 2) = x23;
-            xi = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (; qi < nq; qi += step) {
+        if (qi + step < nq) {
+            load_old(n, qi + step);
+            load_new(n);
         }
-        xi.x = fmaf(alf, p.x, xi.x);
-        xi.y = v1 ? fmaf(alf, p.y, xi.y) : 0.f;
-        xi.z = v2 ? fmaf(alf, p.z, xi.z) : 0.f;
-        xi.w = v3 ? fmaf(alf, p.w, xi.w) : 0.f;
-        r.x = fmaf(-alf, q.x, r.x);
-        r.y = v1 ? fmaf(-alf, q.y, r.y) : 0.f;
-        r.z = v2 ? fmaf(-alf, q.z, r.z) : 0.f;
-        r.w = v3 ? fmaf(-alf, q.w, r.w) : 0.f;
-        *reinterpret_cast<float4*>(a.xinc + o) = xi;
-        *reinterpret_cast<float4*>(a.r + o) = r;
-        acc += (double)r.x * r.x + (double)r.y * r.y + ((double)r.z * r.z + (double)r.w * r.w);
-        qi += (size_t)gridDim.x * kThreads;
-        if (qi < nq) load();
+        const bool v1 = c.x + 1 < W, v2 = c.x + 2 < W, v3 = c.x + 3 < W;
+        if (fold) {
+            double2 x01 = *reinterpret_cast<const double2*>(a.x + c.o);
+            double2 x23 = *reinterpret_cast<const double2*>(a.x + c.o + 2);
+            x01.x += (double)c.xi.x;
+            x01.y = v1 ? x01.y + (double)c.xi.y : 0.0;
+            x23.x = v2 ? x23.x + (double)c.xi.z : 0.0;
+            x23.y = v3 ? x23.y + (double)c.xi.w : 0.0;
+            *reinterpret_cast<double2*>(a.x + c.o) = x01;
+            *reinterpret_cast<double2*>(a.x + c.o + 2) = x23;
+            c.xi = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        c.xi.x = fmaf(alf, c.p.x, c.xi.x);
+        c.xi.y = v1 ? fmaf(alf, c.p.y, c.xi.y) : 0.f;
+        c.xi.z = v2 ? fmaf(alf, c.p.z, c.xi.z) : 0.f;
+        c.xi.w = v3 ? fmaf(alf, c.p.w, c.xi.w) : 0.f;
+        c.r.x = fmaf(-alf, c.q.x, c.r.x);
+        c.r.y = v1 ? fmaf(-alf, c.q.y, c.r.y) : 0.f;
+        c.r.z = v2 ? fmaf(-alf, c.q.z, c.r.z) : 0.f;
+        c.r.w = v3 ? fmaf(-alf, c.q.w, c.r.w) : 0.f;
+        *reinterpret_cast<float4*>(a.xinc + c.o) = c.xi;
+        *reinterpret_cast<float4*>(a.r + c.o) = c.r;
+        acc += (double)c.r.x * c.r.x + (double)c.r.y * c.r.y + ((double)c.r.z * c.r.z + (double)c.r.w * c.r.w);
+        c = n;
     }
     if (LAST) {
         double v[1] = {acc};
@@ -597,9 +609,22 @@ __global__ void __launch_bounds__(kThreads) mg_dense_kernel(Args a)
         for (int q = 0; q < kDenseLoads; ++q) m[q] = lane + 32 * q < n ? __ldg(row + lane + 32 * q) : 0.0;
     };
     load_row();
+    constexpr int NB = (kDenseMax + kThreads - 1) / kThreads;
+    const float* src[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        const int j = min((int)threadIdx.x + k * kThreads, n - 1);
+        src[k] = G.b + (size_t)(j / G.W) * G.P + j % G.W;
+    }
     pdl_wait();
-    if (paused(a.st)) return;
-    for (int j = threadIdx.x; j < n; j += kThreads) b[j] = G.b[(size_t)(j / G.W) * G.P + j % G.W];
+    float bv[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) bv[k] = __ldcg(src[k]);
+    const bool stop = paused(a.st);
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+        if ((int)threadIdx.x + k * kThreads < n) b[threadIdx.x + k * kThreads] = bv[k];
+    if (stop) return;
     __syncthreads();
     for (;;) {
         double s[2] = {0.0, 0.0};
@@ -692,16 +717,11 @@ template <> __device__ __forceinline__ float2 ld2<__nv_bfloat16>(const __nv_bflo
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
 }
 
-// Adds expected TMA bytes to the current phase without arriving; and a plain
-// arrival (the phase completes once its bytes have landed).
+// Adds expected TMA bytes to the current phase without arriving.
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes)
 {
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_only(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // Waits for a TMA stage with a wall-clock limit (2 s); on expiry the solve
@@ -761,16 +781,11 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
             mbar_expect_tx(&full[k], (uint32_t)LY::PB);
             issue_planes(t0 + k * G, k);
         }
-    pdl_enter();
     State* st = a.st;
-    // One thread looks: the lead CTA of this kernel may set need_replace or done
-    // while others start, and a CTA has to take one path.
-    __shared__ int s_stop;
-    if (tid == 0) s_stop = paused(st);
-    __syncthreads();
-    const bool stop = s_stop != 0;
-    const int it = st->iter;
+    // (of FM_SPMV's predecessors only those long complete write iter)
+    const int it = MODE == FM_SPMV ? st->iter : 0;
     const bool first = it == 0;
+    pdl_enter();
     const float om = a.omega, sc = a.scale;
     const CUtensorMap* mv1 = MODE == FM_SPMV ? ((it & 1) ? &tm.m[3] : &tm.m[2]) : &tm.m[2];
     float* pnew = (it & 1) ? a.p0 : a.p1;
@@ -788,30 +803,35 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
         issue_planes(t, s);
         issue_vectors(t, s);
     };
-    auto drain = [&]() {  // complete the requested stages
+    auto drain = [&]() {  // let the requested stages land
         for (int k = 0; k < npre; ++k) stage_wait(&full[k], 0u, st);
     };
-    if (stop) {
-        if (tid == 0)
-            for (int k = 0; k < npre; ++k) mbar_arrive_only(&full[k]);
-        drain();
-        return;
-    }
+    // The vectors are requested before it is known whether there is anything
+    // to do, and the sums of the kernels before are added up while they are on
+    // their way.
     if (tid == 0)
         for (int k = 0; k < npre; ++k) {
             mbar_arrive_expect_tx(&full[k], LY::bytes - (uint32_t)LY::PB);
             issue_vectors(t0 + k * G, k);
         }
-    // Sums of the kernels before, added up while the vectors are on their way.
     float beta = 0.f;
-    if (MODE == FM_SPMV || (MODE == FM_DOWN && pending)) {
-        __shared__ double s_sum;
-        if (tid >= 32 && tid < 64) {
-            const double t = MODE == FM_SPMV ? warp_sum_range(a.parts + (size_t)S_RZ * kMaxParts, 0, a.n_rz)
-                                             : warp_sum_range(a.parts + (size_t)S_RR * kMaxParts, 0, a.n_rr);
-            if (tid == 32) s_sum = t;
-        }
-        __syncthreads();
+    const bool summing = MODE == FM_SPMV || (MODE == FM_DOWN && pending);
+    __shared__ double s_sum;
+    __shared__ int s_stop;
+    if (summing && tid >= 32 && tid < 64) {
+        const double t = MODE == FM_SPMV ? warp_sum_range(a.parts + (size_t)S_RZ * kMaxParts, 0, a.n_rz)
+                                         : warp_sum_range(a.parts + (size_t)S_RR * kMaxParts, 0, a.n_rr);
+        if (tid == 32) s_sum = t;
+    }
+    // One thread looks: the lead CTA of this kernel may set need_replace or done
+    // while others start, and a CTA has to take one path.
+    if (tid == 64) s_stop = paused(st);
+    __syncthreads();
+    if (s_stop) {
+        drain();
+        return;
+    }
+    if (summing) {
         const double sum = s_sum;
         const bool lead = blockIdx.x == 0 && tid == 0;
         if (MODE == FM_SPMV) {
