@@ -543,51 +543,70 @@ __device__ __forceinline__ TRow t_row(const Lev& F, const Lev& C, int i, double 
 // 640 x 480 (300 or 1200), 103.8 / 106.5 / 111.1 at 1080p (510, 510, 2040): one
 // level less costs a row of 2 K doubles per warp, more than its two launches.
 constexpr int kDenseMax = 1300;
-constexpr int kDenseRows = 8;     // rows of M_l per CTA
 
-// Rows kDenseRows * blockIdx.x .. of M_l; thread j forms the entries of column j.
+// M_l from M_{l+1}.  A CTA forms the rows of 8 cells next to each other: their T
+// rows reach 6 x 2 aggregates, whose rows of M_{l+1} it stages in shared
+// memory; thread j applies T to those from the right (12 numbers), then to
+// them from the left, for column j of the 8 rows.  (16 gathers per entry from
+// L2 instead: 54 against 35 us cold for the two levels of 317 x 211.)
+constexpr int kDenseRun = 8;
+constexpr int kDenseParts = 4;  // CTAs per run: 256 columns each at a time
+static int dense_build_smem(int nc) { return 2 * (kDenseRun / 2 + 2) * nc * (int)sizeof(double); }
+
 __global__ void __launch_bounds__(kThreads) mg_dense_build_kernel(Args a, int l)
 {
     pdl_enter();
-    __shared__ TRow rows[kDenseRows];
+    constexpr int NX = kDenseRun / 2 + 2;
+    extern __shared__ __align__(16) unsigned char smem[];
+    double* Ms = reinterpret_cast<double*>(smem);  // [2][NX][nc]
+    __shared__ TRow rows[kDenseRun];
     const Lev& F = a.lev[l];
     const Lev& C = a.lev[l + 1];
-    const int n = F.W * F.H, nc = C.W * C.H;
+    const int n = F.W * F.H, nc = C.W * C.H, runs = (F.W + kDenseRun - 1) / kDenseRun;
     const double om = (double)a.omega, sc = (double)a.scale;
-    const double* Mc = C.M;
     const float* c = static_cast<const float*>(F.c);
-    for (int i0 = blockIdx.x * kDenseRows; i0 < n; i0 += gridDim.x * kDenseRows) {
-        if (threadIdx.x < kDenseRows && i0 + (int)threadIdx.x < n) rows[threadIdx.x] = t_row(F, C, i0 + threadIdx.x, om);
+    for (int item = blockIdx.x; item < runs * F.H * kDenseParts; item += gridDim.x) {
+        const int run = item / kDenseParts, part = item % kDenseParts;
+        const int x0 = (run % runs) * kDenseRun, y = run / runs, X0 = x0 >> 1, Y = y >> 1;
+        const int Ys = min(max(Y + ((y & 1) ? 1 : -1), 0), C.H - 1);
+        const int cells = min(kDenseRun, F.W - x0);
         __syncthreads();
-        for (int j = threadIdx.x; j < n; j += kThreads) {
+        for (int e = 0; e < 2 * NX; ++e) {
+            const int X = min(max(X0 - 1 + e % NX, 0), C.W - 1);
+            const double* src = C.M + (size_t)((e < NX ? Y : Ys) * C.W + X) * nc;
+            for (int j = threadIdx.x; j < nc; j += kThreads) Ms[e * nc + j] = src[j];
+        }
+        if ((int)threadIdx.x < cells) rows[threadIdx.x] = t_row(F, C, y * F.W + x0 + threadIdx.x, om);
+        __syncthreads();
+        for (int j = part * kThreads + threadIdx.x; j < n; j += kDenseParts * kThreads) {
             const TRow tj = t_row(F, C, j, om);
-            const int xj = j % F.W, yj = j / F.W;
+            double u[2 * NX];
+#pragma unroll
+            for (int e = 0; e < 2 * NX; ++e) {
+                const double* row = Ms + e * nc;
+                u[e] = tj.w[0] * row[tj.I[0]] + tj.w[1] * row[tj.I[1]] + tj.w[2] * row[tj.I[2]] + tj.w[3] * row[tj.I[3]];
+            }
+            const int xj = j % F.W, yj = j / F.W, dv = yj - y;
             const size_t oj = (size_t)yj * F.P + xj;
             const double dj = F.Di[oj];
-            for (int q = 0; q < kDenseRows && i0 + q < n; ++q) {
-                const int i = i0 + q, xi = i % F.W, yi = i / F.W;
-                double v = 0.0;
-    #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const double* row = Mc + (size_t)rows[q].I[e] * nc;
-                    v += rows[q].w[e] * (tj.w[0] * row[tj.I[0]] + tj.w[1] * row[tj.I[1]] + tj.w[2] * row[tj.I[2]] +
-                                         tj.w[3] * row[tj.I[3]]);
-                }
-                v *= sc;
-                const int du = xj - xi, dv = yj - yi;
-                if (i == j) v += om * (2.0 - om) * dj;
+#pragma unroll
+            for (int q = 0; q < kDenseRun; ++q) {
+                if (q >= cells) break;
+                const int own = 1 + q / 2, side = (q & 1) ? 2 + q / 2 : q / 2;  // x0 is even
+                double v = sc * (rows[q].w[0] * u[own] + rows[q].w[1] * u[side] + rows[q].w[2] * u[NX + own] +
+                                 rows[q].w[3] * u[NX + side]);
+                const int xi = x0 + q, du = xj - xi;
+                if (du == 0 && dv == 0) v += om * (2.0 - om) * dj;
                 else if (du >= -1 && du <= 1 && dv >= -1 && dv <= 1) {
                     // the coupling is stored at the upper end of the pair: planes E, SW, S, SE
                     const bool up = dv > 0 || (dv == 0 && du > 0);
                     const int k = dv == 0 ? 0 : 2 + (up ? du : -du);
-                    const size_t oi = (size_t)yi * F.P + xi;
-                    const double w = c[(size_t)k * F.ps + (up ? oi : oj)];
-                    v += om * om * w * (double)F.Di[oi] * dj;
+                    const size_t oi = (size_t)y * F.P + xi;
+                    v += om * om * (double)c[(size_t)k * F.ps + (up ? oi : oj)] * (double)F.Di[oi] * dj;
                 }
-                F.M[(size_t)i * n + j] = v;
+                F.M[(size_t)(y * F.W + xi) * n + j] = v;
             }
         }
-        __syncthreads();
     }
 }
 
@@ -993,130 +1012,209 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
 // Set-up kernels
 // ---------------------------------------------------------------------------
 
-// Galerkin coarsening of level l into l+1, one thread per coarse cell: the
-// couplings of the cell's (up to 4) fine cells in both directions are
-// summed per neighbouring aggregate (FP64), in a fixed order.
-template <class S, class T>
-__global__ void mg_build_kernel(Args a, int l, const float* fine_gamma, int gpitch)
+// Galerkin coarsening, one thread per coarse cell: the couplings of the cell's
+// (up to 4) fine cells in both directions are summed per neighbouring
+// aggregate (FP64), in a fixed order.  weight(k, dir, bq, aq) is the coupling
+// of plane k of fine cell (2 X + aq, 2 Y + bq) towards its upper (dir 0) or
+// lower (dir 1) neighbour, 0 where there is none.
+template <class S, class F>
+__device__ __forceinline__ void coarsen(const Lev& C, int X, int Y, double gam, F weight)
 {
-    pdl_enter();
-    const Lev& F = a.lev[l];
-    const Lev& C = a.lev[l + 1];
-    const T* w = static_cast<const T*>(F.c);
-    const int n = C.W * C.H;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int X = i % C.W, Y = i / C.W;
-        double c[4] = {0.0, 0.0, 0.0, 0.0};
-        double ext = 0.0, gam = 0.0;
-        for (int bq = 0; bq < 2; ++bq)
-            for (int aq = 0; aq < 2; ++aq) {
-                const int x = 2 * X + aq, y = 2 * Y + bq;
-                if (x >= F.W || y >= F.H) continue;
-                gam += fine_gamma[(size_t)y * gpitch + x];
-                for (int k = 0; k < S::NP; ++k)
-                    for (int dir = 0; dir < 2; ++dir) {
-                        const int du = dir ? -S::du(k) : S::du(k), dv = dir ? -S::dv(k) : S::dv(k);
-                        const int xj = x + du, yj = y + dv;
-                        if (xj < 0 || xj >= F.W || yj < 0 || yj >= F.H) continue;
-                        // the coupling is stored at the upper end of the pair
-                        const int xs = dir ? xj : x, ys = dir ? yj : y;
-                        const double wv = tof(w[(size_t)k * F.ps + (size_t)ys * F.P + xs]);
-                        const int ox = (xj >> 1) - X, oy = (yj >> 1) - Y;
-                        if (ox == 0 && oy == 0) continue;
-                        ext += wv;
-                        for (int o = 0; o < 4; ++o)
-                            if (ox == CoarseSten::du(o) && oy == CoarseSten::dv(o)) c[o] += wv;
-                    }
-            }
-        const size_t oc = (size_t)Y * C.P + X;
-        float* cp = static_cast<float*>(C.c);
-        for (int o = 0; o < 4; ++o) cp[(size_t)o * C.ps + oc] = (float)c[o];
-        C.gam[oc] = (float)gam;
-        C.D[oc] = (float)(gam + ext);
-        C.Di[oc] = gam + ext > 0.0 ? (float)(1.0 / (gam + ext)) : 0.f;
-    }
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    double ext = 0.0;
+#pragma unroll
+    for (int bq = 0; bq < 2; ++bq)
+#pragma unroll
+        for (int aq = 0; aq < 2; ++aq)
+#pragma unroll
+            for (int k = 0; k < S::NP; ++k)
+#pragma unroll
+                for (int dir = 0; dir < 2; ++dir) {
+                    const int du = dir ? -S::du(k) : S::du(k), dv = dir ? -S::dv(k) : S::dv(k);
+                    const int ox = (aq + du) >> 1, oy = (bq + dv) >> 1;  // aggregate of the neighbour, from (X, Y)
+                    if (ox == 0 && oy == 0) continue;
+                    const double wv = weight(k, dir, bq, aq);
+                    ext += wv;
+#pragma unroll
+                    for (int o = 0; o < 4; ++o)
+                        if (ox == CoarseSten::du(o) && oy == CoarseSten::dv(o)) c[o] += wv;
+                }
+    const size_t oc = (size_t)Y * C.P + X;
+    float* cp = static_cast<float*>(C.c);
+#pragma unroll
+    for (int o = 0; o < 4; ++o) cp[(size_t)o * C.ps + oc] = (float)c[o];
+    C.gam[oc] = (float)gam;
+    C.D[oc] = (float)(gam + ext);
+    C.Di[oc] = gam + ext > 0.0 ? (float)(1.0 / (gam + ext)) : 0.f;
 }
 
-// Dense FP64 inverse of the coarsest operator by in-place Gauss-Jordan
-// elimination (SPD: no pivoting), one CTA, matrix in shared memory.
-__global__ void __launch_bounds__(kThreads) mg_inverse_kernel(Args a)
+// Summed scribble weight of a coarse cell's fine cells.
+__device__ __forceinline__ double gamma_sum(const Lev& F, const float* g, int gp, int X, int Y)
+{
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int x = 2 * X + (q & 1), y = 2 * Y + (q >> 1);
+        if (x < F.W && y < F.H) t += g[(size_t)y * gp + x];
+    }
+    return t;
+}
+
+// Level 0 into level 1: tiles of 32 x 8 coarse cells, whose 64 x 16 pixels of
+// the 12 planes (with the halo of the mirrored couplings) go through shared
+// memory, so that the planes are read once and coalesced (1080p, FP16: 143 us
+// cold with each thread loading its own 96 couplings, 28 now, 9 us at the copy
+// rate).
+constexpr int kBuildTY = 16;
+template <class T>
+__global__ void __launch_bounds__(kThreads) mg_build0_kernel(Args a)
 {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smem[];
+    T* pt = reinterpret_cast<T*>(smem);
+    const Lev& F = a.lev[0];
+    const Lev& C = a.lev[1];
+    const int cx = threadIdx.x & 31, cy = threadIdx.x >> 5;
+    const int tiles_x = (F.W + kTX - 1) / kTX, tiles = tiles_x * ((F.H + kBuildTY - 1) / kBuildTY);
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int x0 = (t % tiles_x) * kTX, y0 = (t / tiles_x) * kBuildTY;
+        __syncthreads();
+        load_planes<T, FineSten::NP, kBuildTY + kHalo>(pt, static_cast<const T*>(F.c), F.ps, F.P, F.W, F.H, x0, y0);
+        const int X = (x0 >> 1) + cx, Y = (y0 >> 1) + cy;
+        const double gam = gamma_sum(F, a.gamma, a.P, X, Y);
+        __syncthreads();
+        if (X < C.W && Y < C.H)
+            coarsen<FineSten>(C, X, Y, gam, [&](int k, int dir, int bq, int aq) {
+                const int lx = 2 * cx + aq + 8 - (dir ? FineSten::du(k) : 0);
+                const int ly = 2 * cy + bq + kHalo - (dir ? FineSten::dv(k) : 0);
+                return (double)tof(pt[((size_t)k * (kBuildTY + kHalo) + ly) * kPW + lx]);
+            });
+    }
+}
+
+// Level l >= 1 into l + 1, one cell.
+__device__ __forceinline__ void coarsen_cell(const Args& a, int l, int i)
+{
+    const Lev& F = a.lev[l];
+    const Lev& C = a.lev[l + 1];
+    const float* w = static_cast<const float*>(F.c);
+    const int X = i % C.W, Y = i / C.W;
+    coarsen<CoarseSten>(C, X, Y, gamma_sum(F, F.gam, F.P, X, Y), [&](int k, int dir, int bq, int aq) {
+        const int du = CoarseSten::du(k), dv = CoarseSten::dv(k);
+        const int x = 2 * X + aq, y = 2 * Y + bq;
+        const int xn = dir ? x - du : x + du, yn = dir ? y - dv : y + dv;
+        const bool in = x < F.W && y < F.H && xn >= 0 && xn < F.W && yn >= 0 && yn < F.H;
+        return in ? (double)w[(size_t)k * F.ps + (dir ? (size_t)yn * F.P + xn : (size_t)y * F.P + x)] : 0.0;
+    });
+}
+
+__global__ void __launch_bounds__(128) mg_build_kernel(Args a, int l)
+{
+    pdl_enter();
+    const Lev& C = a.lev[l + 1];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.W * C.H; i += gridDim.x * blockDim.x) coarsen_cell(a, l, i);
+}
+
+// The levels after lb in one CTA (each depends on the one before), then the
+// dense FP64 inverse of the coarsest operator by Gauss-Jordan elimination (SPD:
+// no pivoting).  The matrix stays in registers: thread (row, sub) holds the
+// columns sub, sub + 8, ...; a step publishes the pivot's row and column and its
+// reciprocal in shared memory (two copies in turn, so one barrier a step).
+// Bound by the chain of one step (FP64 reciprocal, barrier, update: 0.45-0.6 us);
+// with the matrix in shared memory, two barriers and an index division per
+// entry it was 1.2 us for n = 40 and 2.8 for n = 70.
+// NC: columns per thread, 8 NC >= n; 8 n threads, rounded up to a warp.
+constexpr int kOneCtaCells = 1024;  // a level this small is built by one CTA
+template <int NC>
+__global__ void __launch_bounds__(64 * NC) mg_coarse_kernel(Args a, int lb)
+{
+    pdl_enter();
+    for (int l = lb; l < a.L; ++l) {
+        for (int i = threadIdx.x; i < a.lev[l + 1].W * a.lev[l + 1].H; i += blockDim.x) coarsen_cell(a, l, i);
+        __syncthreads();
+    }
+    __shared__ double s_row[2][kCoarseMax], s_col[2][kCoarseMax];
+    __shared__ double s_inv[2], s_dmax;
     const Lev& C = a.lev[a.L];
-    const int n = C.W * C.H;
-    double* A = reinterpret_cast<double*>(smem);
-    double* row = A + (size_t)n * n;
-    double* col = row + kCoarseMax;
-    __shared__ int s_bad;
-    for (int i = threadIdx.x; i < n * n; i += kThreads) A[i] = 0.0;
-    if (threadIdx.x == 0) s_bad = 0;
-    __syncthreads();
+    const int n = C.W * C.H, row = threadIdx.x >> 3, sub = threadIdx.x & 7;
     const float* cp = static_cast<const float*>(C.c);
-    for (int I = threadIdx.x; I < n; I += kThreads) {
-        const int X = I % C.W, Y = I / C.W;
-        const size_t o = (size_t)Y * C.P + X;
-        A[(size_t)I * n + I] = C.D[o];
-        for (int k = 0; k < 4; ++k) {
-            const int Xj = X + CoarseSten::du(k), Yj = Y + CoarseSten::dv(k);
-            if (Xj < 0 || Xj >= C.W || Yj >= C.H) continue;
-            const int J = Yj * C.W + Xj;
-            const double v = -(double)cp[(size_t)k * C.ps + o];
-            A[(size_t)I * n + J] = v;
-            A[(size_t)J * n + I] = v;
+    double v[NC];
+    const int xr = row % C.W, yr = row / C.W;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+        const int col = sub + 8 * j, xc = col % C.W, yc = col / C.W, du = xc - xr, dv = yc - yr;
+        v[j] = 0.0;
+        if (row < n && col < n && du >= -1 && du <= 1 && dv >= -1 && dv <= 1) {
+            const size_t orow = (size_t)yr * C.P + xr, ocol = (size_t)yc * C.P + xc;
+            const bool up = dv > 0 || (dv == 0 && du > 0);
+            const int k = dv == 0 ? 0 : 2 + (up ? du : -du);
+            v[j] = row == col ? (double)C.D[orow] : -(double)cp[(size_t)k * C.ps + (up ? orow : ocol)];
         }
     }
-    __syncthreads();
     // Zero rows (aggregates with no coupling and no scribble weight, as in
     // images less than 3 pixels wide or tall, where no 3x3 window exists) are
     // left out: for a positive semidefinite matrix a zero pivot means a zero
     // row and column, and the inverse on the remaining rows is exact.
-    double dmax = 0.0;
-    for (int i = 0; i < n; ++i) dmax = fmax(dmax, A[(size_t)i * n + i]);
-    for (int k = 0; k < n; ++k) {
-        const double piv = A[(size_t)k * n + k];
-        if (!isfinite(piv) || piv < 0.0) {
-            if (threadIdx.x == 0) s_bad = 1;
-            break;
-        }
-        if (piv <= 1e-300 + 1e-14 * dmax) {
-            for (int j = threadIdx.x; j < n; j += kThreads) {
-                A[(size_t)k * n + j] = 0.0;
-                A[(size_t)j * n + k] = 0.0;
-            }
-            __syncthreads();
-            continue;
-        }
-        const double inv = 1.0 / piv;
-        for (int j = threadIdx.x; j < n; j += kThreads) {
-            row[j] = A[(size_t)k * n + j] * inv;
-            col[j] = A[(size_t)j * n + k];
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < n * n; e += kThreads) {
-            const int i = e / n, j = e % n;
-            double v;
-            if (i == k && j == k) v = inv;
-            else if (i == k) v = row[j];
-            else if (j == k) v = -col[i] * inv;
-            else v = A[e] - col[i] * row[j];
-            A[e] = v;
-        }
-        __syncthreads();
+    if (threadIdx.x < 32) {
+        double m = 0.0;
+        for (int i = threadIdx.x; i < n; i += 32) m = fmax(m, (double)C.D[(size_t)(i / C.W) * C.P + i % C.W]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (threadIdx.x == 0) s_dmax = m;
     }
     __syncthreads();
-    if (s_bad) {
+    const double tiny = 1e-300 + 1e-14 * s_dmax;
+    bool bad = false;
+#pragma unroll
+    for (int jb = 0; jb < NC; ++jb) {
+        for (int m = 0; m < 8; ++m) {
+            const int k = 8 * jb + m;
+            if (k >= n || bad) break;
+            double* pr = s_row[m & 1];
+            double* pc = s_col[m & 1];
+            if (row == k) {
+#pragma unroll
+                for (int j = 0; j < NC; ++j) pr[sub + 8 * j] = v[j];
+                if (sub == m) {
+                    const double piv = v[jb];
+                    const bool fine = isfinite(piv) && piv >= 0.0;
+                    s_inv[m & 1] = !fine ? -1.0 : (piv <= tiny ? 0.0 : 1.0 / piv);
+                }
+            }
+            if (sub == m) pc[row] = v[jb];
+            __syncthreads();
+            const double inv = s_inv[m & 1];  // 0: a zero row, -1: not positive semidefinite
+            if (inv < 0.0) {
+                bad = true;
+                break;
+            }
+            if (row == k) {
+#pragma unroll
+                for (int j = 0; j < NC; ++j) v[j] *= inv;
+                if (sub == m) v[jb] = inv;
+            } else {
+                const double f = pc[row] * inv;
+#pragma unroll
+                for (int j = 0; j < NC; ++j) v[j] = fma(-f, pr[sub + 8 * j], v[j]);
+                if (sub == m) v[jb] = -f;
+            }
+        }
+    }
+    if (bad) {
         if (threadIdx.x == 0) {
             a.st->status = GM_ERR_BREAKDOWN;
             a.st->done = 1;
         }
         return;
     }
-    for (int e = threadIdx.x; e < n * n; e += kThreads) C.M[e] = A[e];
+#pragma unroll
+    for (int j = 0; j < NC; ++j)
+        if (row < n && sub + 8 * j < n) C.M[(size_t)row * n + sub + 8 * j] = v[j];
 }
 
-// 1 / d of the level-0 iteration diagonal (0 where d = 0).
-__global__ void mg_diag0_kernel(Args a)
+// 1 / d of the level-0 iteration diagonal (0 where d = 0), FP64 solution from
+// the FP32 guess (none: only the hierarchy is set up), initial state.
+__global__ void mg_init_kernel(Args a)
 {
     pdl_enter();
     const int W = a.W, H = a.H, P = a.P;
@@ -1125,19 +1223,10 @@ __global__ void mg_diag0_kernel(Args a)
         const size_t o = (i / W) * P + i % W;
         const float d = a.lev[0].D[o];
         a.lev[0].Di[o] = d > 0.f ? 1.f / d : 0.f;
-    }
-}
-
-// Initial state, FP64 solution from the FP32 guess.
-__global__ void mg_init_kernel(Args a)
-{
-    pdl_enter();
-    const int W = a.W, H = a.H, P = a.P;
-    const size_t n = (size_t)W * H;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int y = (int)(i / W), x = (int)(i % W);
-        a.x[(size_t)y * P + x] = (double)a.alpha_in[(size_t)y * W + x];
-        a.xinc[(size_t)y * P + x] = 0.f;
+        if (a.alpha_in) {
+            a.x[o] = (double)a.alpha_in[i];
+            a.xinc[o] = 0.f;
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         State* st = a.st;
@@ -1146,7 +1235,7 @@ __global__ void mg_init_kernel(Args a)
         st->iter_next = 0;
         st->done = 0;
         st->status = GM_OK;
-        st->need_replace = 1;
+        st->need_replace = a.alpha_in ? 1 : 0;
         st->replacements = 0;
         st->fold_at = -1;
         st->restart_at = -1;
@@ -1504,26 +1593,23 @@ struct Enq {
         go(mg_replace_kernel, tiles_of(a.W, a.H, kTY), sm, kThreads, a);
     }
 
-    void build() const
-    {
-        go(mg_diag0_kernel, pointwise_tiles() * 4, 0, kThreads, a);
-        for (int l = 0; l < a.L; ++l) {
-            const Lev& C = a.lev[l + 1];
-            const int t = (C.W * C.H + 127) / 128;
-            if (l == 0) go(mg_build_kernel<FineSten, T>, t, 0, 128, a, 0, (const float*)a.gamma, a.P);
-            else go(mg_build_kernel<CoarseSten, float>, t, 0, 128, a, l, (const float*)a.lev[l].gam, a.lev[l].P);
-        }
-        const int n = a.lev[a.L].W * a.lev[a.L].H;
-        const int sm = (int)(sizeof(double) * ((size_t)n * n + 2 * kCoarseMax));
-        go(mg_inverse_kernel, 1, sm, kThreads, a);
-        for (int l = a.L - 1; l >= a.lt; --l)
-            go(mg_dense_build_kernel, (a.lev[l].W * a.lev[l].H + kDenseRows - 1) / kDenseRows, 0, kThreads, a, l);
-    }
-
     void setup() const
     {
         go(mg_init_kernel, pointwise_tiles(), 0, kThreads, a);
-        build();
+        constexpr int sm0 = (int)sizeof(T) * FineSten::NP * (kBuildTY + kHalo) * kPW;
+        go(mg_build0_kernel<T>, tiles_of(a.W, a.H, kBuildTY), sm0, kThreads, a);
+        int l = 1;
+        for (; l < a.L && (long long)a.lev[l + 1].W * a.lev[l + 1].H > kOneCtaCells; ++l)
+            go(mg_build_kernel, (a.lev[l + 1].W * a.lev[l + 1].H + 127) / 128, 0, 128, a, l);
+        const int nc = a.lev[a.L].W * a.lev[a.L].H, threads = (8 * nc + 31) / 32 * 32;
+        static_assert(kCoarseMax == 128, "columns per thread");
+        if (nc <= 40) go(mg_coarse_kernel<5>, 1, 0, threads, a, l);
+        else if (nc <= 64) go(mg_coarse_kernel<8>, 1, 0, threads, a, l);
+        else if (nc <= 96) go(mg_coarse_kernel<12>, 1, 0, threads, a, l);
+        else go(mg_coarse_kernel<16>, 1, 0, threads, a, l);
+        for (l = a.L - 1; l >= a.lt; --l)
+            go(mg_dense_build_kernel, (a.lev[l].W + kDenseRun - 1) / kDenseRun * a.lev[l].H * kDenseParts,
+               dense_build_smem(a.lev[l + 1].W * a.lev[l + 1].H), kThreads, a, l);
     }
 
     // One loop pass of preconditioner, matrix product and update; an iteration
@@ -2083,11 +2169,10 @@ extern "C" int gm_levin_mg_inspect(const gm_levin_store* store, int use_low, con
     FineMaps fm;
     GM_TRY(make_maps(a, tcode ? 2 : 4, tcode_dtype(tcode), fm));
     cudaStream_t st = (cudaStream_t)stream;
-    GM_CUDA_TRY(cudaMemsetAsync(a.st, 0, sizeof(State), st));
     auto go = [&](auto tag) {
         using T = decltype(tag);
         Enq<T> q{a, sms, st, false, &fm};
-        q.build();
+        q.setup();
         if (r && z) {
             cudaMemcpy2DAsync(a.r, (size_t)a.P * 4, r, (size_t)a.W * 4, (size_t)a.W * 4, a.H, cudaMemcpyDeviceToDevice,
                               st);
