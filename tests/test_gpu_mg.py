@@ -66,10 +66,13 @@ def test_vcycle_matches_oracle(orc, prec):
     assert err <= 1e-4, err
 
 
-@pytest.mark.parametrize("W,H", [(16, 15), (17, 16), (23, 3), (72, 72), (73, 72), (145, 37), (80, 131), (300, 17)])
+@pytest.mark.parametrize("W,H", [(16, 15), (17, 16), (23, 3), (72, 72), (73, 72), (145, 37), (80, 131), (300, 17),
+                                 (171, 131), (402, 283), (1300, 21)])
 def test_vcycle_dense_level_shapes(orc, W, H):
-    """Sizes around the dense level's limits: the coarsest level alone, levels of
-    just under and just over its cell limit, odd sides.  Tolerance: the parity
+    """Sizes around the limits of the dense level and of the two-level kernels: the
+    coarsest level alone, levels of
+    just under and just over the cell limit, one pair of levels, a pair below a
+    single level, odd sides and thin images.  Tolerance: the parity
     bar of the FP32 V-cycle (1e-4)."""
     torch = torch_cuda()
     st, p, w, g, b = _store(orc, W, H, "fp16", seed=4)
