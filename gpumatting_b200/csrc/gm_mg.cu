@@ -169,46 +169,30 @@ __device__ __forceinline__ void pdl_enter()
     pdl_trigger();
 }
 
-// Plane tile: NP planes x ROWS rows (y0 - 2 .. y0 + ROWS - 3) x kPW columns
-// starting at x0 - 8 (16-byte aligned: x0 is a multiple of 64 and P of 8).
-// Elements outside the W x H level read as zero.  Every thread issues all of
-// its 16-byte loads before the first shared-memory store, so a tile's loads
-// are in flight together.
+// Starts copying a plane tile: NP planes x ROWS rows (y0 - 2 .. y0 + ROWS - 3) x
+// kPW columns starting at x0 - 8 (16-byte aligned: x0 is a multiple of 64 and P
+// of 8).  Elements outside the W x H level read as zero (a partial copy fills
+// with zeros).  All of a tile's copies are in flight together.
 template <class T, int NP, int ROWS>
 __device__ __forceinline__ void load_planes(T* sm, const T* g, size_t ps, int P, int W, int H, int x0, int y0)
 {
     constexpr int EPV = 16 / sizeof(T);
     constexpr int VPR = kPW / EPV;
     constexpr int TOTAL = NP * ROWS * VPR;
-    constexpr int ITER = (TOTAL + kThreads - 1) / kThreads;
-    constexpr int CH = 6;  // loads in flight per thread (registers: 4 per load)
 #pragma unroll
-    for (int j0 = 0; j0 < ITER; j0 += CH) {
-        uint4 val[CH];
-#pragma unroll
-        for (int j = 0; j < CH; ++j) {
-            const int i = threadIdx.x + (j0 + j) * kThreads;
-            const int v = i % VPR, r = (i / VPR) % ROWS, k = i / (VPR * ROWS);
-            const int gx = x0 - 8 + v * EPV, gy = y0 - kHalo + r;
-            val[j] = make_uint4(0u, 0u, 0u, 0u);
-            if (j0 + j < ITER && i < TOTAL && gy >= 0 && gy < H && gx >= 0 && gx < W)
-                val[j] = __ldg(reinterpret_cast<const uint4*>(g + (size_t)k * ps + (size_t)gy * P + gx));
-        }
-#pragma unroll
-        for (int j = 0; j < CH; ++j) {
-            const int i = threadIdx.x + (j0 + j) * kThreads;
-            if (j0 + j < ITER && i < TOTAL) {
-                const int v = i % VPR;
-                const int gx = x0 - 8 + v * EPV;
-                T* dst = sm + (size_t)(i / VPR) * kPW + v * EPV;
-                *reinterpret_cast<uint4*>(dst) = val[j];
-                if (gx + EPV > W && gx < W) {
-                    for (int e = W - gx; e < EPV; ++e) dst[e] = T(0.0f);
-                }
-            }
-        }
+    for (int j = 0; j < (TOTAL + kThreads - 1) / kThreads; ++j) {
+        const int i = threadIdx.x + j * kThreads;
+        const int v = i % VPR, r = (i / VPR) % ROWS, k = i / (VPR * ROWS);
+        const int gx = x0 - 8 + v * EPV, gy = y0 - kHalo + r;
+        const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
+        const int bytes = in ? min(EPV, W - gx) * (int)sizeof(T) : 0;
+        if (i < TOTAL)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sm + (size_t)(i / VPR) * kPW + v * EPV)),
+                         "l"(g + (in ? (size_t)k * ps + (size_t)gy * P + gx : 0)), "r"(bytes)
+                         : "memory");
     }
 }
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // Deterministic grid reductions: each CTA publishes its partial sums, the
@@ -385,8 +369,11 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
 }
 
 // True residual r = b - A x with the FP32 planes in FP64 arithmetic (runs
-// only when a replacement is due).  Also forms ||b||^2 on the first call.
-__global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
+// only when a replacement is due).  Four CTAs per SM hide one tile's loads
+// behind the others' arithmetic: 62 us at 1080p, 452 at 4096^2 (with 3 CTAs, or
+// with gamma and b loaded where they are used, 73 and 560; 92 B per pixel take
+// 29 and 235).  Also forms ||b||^2 on the first call.
+__global__ void __launch_bounds__(kThreads, 4) mg_replace_kernel(Args a)
 {
     pdl_enter();
     State* st = a.st;
@@ -417,11 +404,21 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
             const size_t o = (size_t)gy * P + gx;
             xv[j] = (i < XT && gx >= 0 && gx < W && gy >= 0 && gy < H) ? a.x[o] + (double)a.xinc[o] : 0.0;
         }
+        // the pixels' own values, in flight with the rest
+        float gv[2], bw[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int gx = x0 + tx + 32 * h, gy = y0 + ty;
+            const bool in = gx < W && gy < H;
+            gv[h] = in ? a.gamma[(size_t)gy * P + gx] : 0.f;
+            bw[h] = in ? a.bvec[(size_t)gy * a.bpitch + gx] : 0.f;
+        }
 #pragma unroll
         for (int j = 0; j < XI; ++j) {
             const int i = threadIdx.x + j * kThreads;
             if (i < XT) xt[i] = xv[j];
         }
+        copies_done();
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -430,7 +427,7 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
                 const size_t o = (size_t)gy * P + gx;
                 const int vc = (ty + kHalo) * kVW + lx + kHalo;
                 const double xc = xt[vc];
-                double y = (double)a.gamma[o] * xc;
+                double y = (double)gv[h] * xc;
 #pragma unroll
                 for (int k = 0; k < FineSten::NP; ++k) {
                     const int du = FineSten::du(k), dv = FineSten::dv(k);
@@ -438,7 +435,7 @@ __global__ void __launch_bounds__(kThreads, 3) mg_replace_kernel(Args a)
                     const double wl = pt[((size_t)k * (kTY + kHalo) + ty + kHalo - dv) * kPW + lx + 8 - du];
                     y += wu * (xc - xt[vc + dv * kVW + du]) + wl * (xc - xt[vc - dv * kVW - du]);
                 }
-                const double bv = a.bvec[(size_t)gy * a.bpitch + gx];
+                const double bv = bw[h];
                 const double r = bv - y;
                 a.r[o] = (float)r;
                 rr += r * r;
@@ -1038,7 +1035,6 @@ __device__ __forceinline__ void stage(float* dst, const float* g, int P, int W, 
                          : "memory");
     }
 }
-__device__ __forceinline__ void stage_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // S = sum_j w_ij v_j at index i of rows of RW cells; the planes are RC cells apart.
 template <int RW, int RC>
@@ -1099,7 +1095,7 @@ __global__ void __launch_bounds__(kPairThreads) mg_pair_down_kernel(Args a, int 
             bf[j] = i < FW * FH && x >= 0 && x < F.W && y >= 0 && y < F.H ? __ldcg(F.b + (size_t)y * F.P + x) : 0.f;
         }
         if (paused(a.st)) {
-            stage_done();
+            copies_done();
             return;
         }
 #pragma unroll
@@ -1110,7 +1106,7 @@ __global__ void __launch_bounds__(kPairThreads) mg_pair_down_kernel(Args a, int 
                 rb[i] = rho_of(bf[j], df[j], om, 0.f);
             }
         }
-        stage_done();
+        copies_done();
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < NM; ++j) {
@@ -1188,7 +1184,7 @@ __global__ void __launch_bounds__(kPairThreads) mg_pair_up_kernel(Args a, int l)
             xc[j] = i < YW * YH && x >= 0 && x < G.W && y >= 0 && y < G.H ? __ldcg(C.x + (size_t)(y >> 1) * C.P + (x >> 1))
                                                                           : 0.f;
         }
-        stage_done();
+        copies_done();
         if (paused(a.st)) return;
 #pragma unroll
         for (int j = 0; j < NY; ++j) {  // (each thread reads what it staged itself)
@@ -1294,6 +1290,7 @@ __global__ void __launch_bounds__(kThreads) mg_build0_kernel(Args a)
         load_planes<T, FineSten::NP, kBuildTY + kHalo>(pt, static_cast<const T*>(F.c), F.ps, F.P, F.W, F.H, x0, y0);
         const int X = (x0 >> 1) + cx, Y = (y0 >> 1) + cy;
         const double gam = gamma_sum(F, a.gamma, a.P, X, Y);
+        copies_done();
         __syncthreads();
         if (X < C.W && Y < C.H)
             coarsen<FineSten>(C, X, Y, gam, [&](int k, int dir, int bq, int aq) {
