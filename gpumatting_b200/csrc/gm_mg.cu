@@ -142,7 +142,7 @@ struct Args {
     double rtol;
     int max_iters, replace_every;
     int outer_low;  // the level-0 SpMV streams the FP16 iteration planes, not w32
-    int spare;
+    int rows0;      // tile rows of the level-0 kernels on 2-byte planes
     float omega, scale;
     // conditional-node handles (0 = host-driven loop): the loop over iterations
     // up to the next residual replacement, and the loop over replacements
@@ -689,13 +689,16 @@ struct TMaps {
     CUtensorMap m[5];
 };
 
-__host__ __device__ constexpr int fine_rows(int esize) { return esize == 2 ? 16 : 8; }
+// Tile rows of the TMA kernels: 8 with 4-byte planes (two CTAs per SM fit); with
+// the 2-byte planes of level 0, 16 (one CTA per SM, a smaller share of halo rows) or
+// 8, chosen per solve by level0_rows.
+constexpr int kRows = 8, kTallRows = 16;
 __host__ __device__ constexpr int b128(int x) { return (x + 127) & ~127; }
 
-template <int MODE, int ES, int NP = 12>
+template <int MODE, int ES, int NP, int ROWS>
 struct FineLayout {
-    static constexpr int TH = fine_rows(ES);
-    static constexpr int THR = ES == 2 ? 512 : 256;  // threads: 64 column pairs x TH / 2 row pairs
+    static constexpr int TH = ROWS;
+    static constexpr int THR = 32 * TH;  // threads: 64 column pairs x TH / 2 row pairs
     static constexpr int PB = NP * (TH + 2) * kFBW * ES;
     static constexpr int VB = (TH + 4) * kFBW * 4;
     static constexpr int XB = MODE == FM_UP ? (TH / 2 + 2) * kXBW * 4 : 0;
@@ -705,9 +708,8 @@ struct FineLayout {
     static constexpr int x_off = v1_off + b128(VB);
     static constexpr int d_off = x_off + b128(XB);
     static constexpr int stage = d_off + b128(DB);
-    static constexpr int vt_off = 2 * stage;
-    static constexpr int bar_off = vt_off + b128(VB);
-    static constexpr int total = bar_off + 64 + 128;  // + room to align the base to 128 bytes
+    // nst stages, the stencil input, the barriers; + room to align the base to 128 bytes
+    static constexpr int total(int nst) { return nst * stage + b128(VB) + 64 + 128; }
     static constexpr uint32_t bytes = (uint32_t)(PB + 2 * VB + XB + DB);
 };
 
@@ -757,13 +759,13 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar, uint32_t parity, State
     return true;
 }
 
-template <int MODE, class S, class T>
-__global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::NP>::THR, 1)
-    mg_fine_kernel(const __grid_constant__ TMaps tm, Args a, int l, int pending)
+template <int MODE, class S, class T, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS, 1)
+    mg_fine_kernel(const __grid_constant__ TMaps tm, Args a, int l, int nst, int pending)
 {
     constexpr int ES = FinePlanes<MODE, T>::ES;
     using PT = typename FinePlanes<MODE, T>::PT;
-    using LY = FineLayout<MODE, ES, S::NP>;
+    using LY = FineLayout<MODE, ES, S::NP, ROWS>;
     constexpr int TH = LY::TH, NT = LY::THR, RPT = TH / (NT / 64);
     static_assert(RPT == 2, "each thread covers one row pair");
     constexpr int PW = (TH + 2) * kFBW;  // elements per plane in the box
@@ -771,8 +773,8 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
     // the reduction's static shared memory, so align its base by hand.
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + LY::bar_off);
-    float* vt = reinterpret_cast<float*>(smem + LY::vt_off);
+    float* vt = reinterpret_cast<float*>(smem + nst * LY::stage);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + nst * LY::stage + b128(LY::VB));
     const Lev& F = a.lev[l];
     const int W = F.W, H = F.H, P = F.P, tid = threadIdx.x, G = gridDim.x;
     const int ntx = (W + kFTW - 1) / kFTW, ntiles = ntx * ((H + TH - 1) / TH);
@@ -791,7 +793,7 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
     // or the set-up kernels, which completed before this kernel's predecessor
     // began), so the first two stages' plane boxes are requested before the
     // wait for the predecessor; the stage's arrival comes with the vectors.
-    const int npre = (t0 < ntiles ? 1 : 0) + (t0 + G < ntiles ? 1 : 0);
+    const int npre = (t0 < ntiles ? 1 : 0) + (nst > 1 && t0 + G < ntiles ? 1 : 0);
     if (tid == 0)
         for (int k = 0; k < npre; ++k) {
             mbar_expect_tx(&full[k], (uint32_t)LY::PB);
@@ -996,8 +998,8 @@ __global__ void __launch_bounds__(FineLayout<MODE, FinePlanes<MODE, T>::ES, S::N
             }
         }
         __syncthreads();  // every thread is done with stage s and the input tile
-        if (tid == 0 && t + 2 * G < ntiles) issue(t + 2 * G, s);
-        s ^= 1;
+        if (tid == 0 && t + nst * G < ntiles) issue(t + nst * G, s);
+        s ^= nst - 1;
     }
     if (!ok) return;
     static_assert(NT <= 1024, "");
@@ -1675,6 +1677,18 @@ static int outer_low_for(int tcode, double rtol)
     return tcode == 1 && !(rtol > 0.0 && rtol < kOuterLowMinRtol) ? 1 : 0;
 }
 
+// Tile rows of the level-0 kernels on 2-byte planes.  Short tiles spread a small
+// image over more SMs and leave room for a second CTA (the next kernel's, or
+// another solve's) on each; their halo rows (10 of 8 plane rows, 12 of 8 vector
+// rows) cost more L2 and DRAM reads on a large one.  Us per iteration with 16 and 8
+// rows: 20.7 / 19.5 at 317 x 211, 32.6 / 30.7 at 640 x 480, 45 / 45 at 960 x 720 (eight
+// such solves at once 284 / 273 us), 51.8 / 52.6 at 1501 x 703, 500 / 547 at 4096^2.
+static int level0_rows(int W, int H, int sms)
+{
+    const long long tiles = (long long)((W + kFTW - 1) / kFTW) * ((H + kRows - 1) / kRows);
+    return tiles <= 5LL * sms ? kRows : kTallRows;
+}
+
 // Tensor maps of the level-0 kernels (es: bytes per element of the
 // iteration planes).
 static int make_maps(const Args& a, int es, CUtensorMapDataType dt, FineMaps& fm)
@@ -1692,7 +1706,7 @@ static int make_maps(const Args& a, int es, CUtensorMapDataType dt, FineMaps& fm
         const uint32_t b2[2] = {(uint32_t)bw, (uint32_t)bh};
         return gm_make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), d2, s2, b2);
     };
-    const int t32 = fine_rows(4), tlo = fine_rows(es);
+    const int t32 = kRows, tlo = es == 2 ? a.rows0 : kRows;
     const Lev& L0 = a.lev[0];
     // the SpMV streams the FP16 iteration planes and their diagonal d when
     // outer_low is set, else the FP32 planes and d32
@@ -1765,30 +1779,38 @@ struct Enq {
     template <int MODE> void fine(int l, int pending = 0) const
     {
         const TMaps& m = MODE == FM_SPMV ? fm->spmv : (MODE == FM_DOWN ? fm->down[l] : fm->up[l]);
-        with_fine<MODE>(l, [&](auto fn, int tiles, int smem, int threads) { go(fn, tiles, smem, threads, m, a, l, pending); });
+        with_fine<MODE>(l, [&](auto fn, int tiles, int smem, int threads, int nst) {
+            go(fn, tiles, smem, threads, m, a, l, nst, pending);
+        });
     }
 
-    // The kernel and launch shape of one level's pass.
+    // The kernel and launch shape of one level's pass.  One ring stage where
+    // every tile gets a CTA of its own: nothing is left to prefetch, and with
+    // half the shared memory a second CTA (the next kernel's, or another
+    // solve's) fits beside it.
     template <int MODE, class F> auto with_fine(int l, F f) const
     {
         const Lev& G = a.lev[l];
-        auto tiles = [&](int th) { return ((G.W + kFTW - 1) / kFTW) * ((G.H + th - 1) / th); };
-        if (l > 0) {
-            using LY = FineLayout<MODE, 4, 4>;
-            return f(mg_fine_kernel<MODE, CoarseSten, float>, tiles(LY::TH), LY::total, LY::THR);
-        }
-        if (MODE == FM_SPMV && !a.outer_low) {
-            using LY = FineLayout<MODE, 4, 12>;
-            return f(mg_fine_kernel<MODE, FineSten, float>, tiles(LY::TH), LY::total, LY::THR);
-        }
-        using LY = FineLayout<MODE, FinePlanes<MODE, T>::ES, 12>;
-        return f(mg_fine_kernel<MODE, FineSten, T>, tiles(LY::TH), LY::total, LY::THR);
+        auto shape = [&](auto fn, auto layout) {
+            using LY = decltype(layout);
+            const int tiles = ((G.W + kFTW - 1) / kFTW) * ((G.H + LY::TH - 1) / LY::TH);
+            const int nst = tiles <= sms * occupancy((const void*)fn, LY::total(1), LY::THR) ? 1 : 2;
+            return f(fn, tiles, LY::total(nst), LY::THR, nst);
+        };
+        constexpr int ES = FinePlanes<MODE, T>::ES;
+        if (l > 0) return shape(mg_fine_kernel<MODE, CoarseSten, float, kRows>, FineLayout<MODE, 4, 4, kRows>());
+        if (MODE == FM_SPMV && !a.outer_low)
+            return shape(mg_fine_kernel<MODE, FineSten, float, kRows>, FineLayout<MODE, 4, 12, kRows>());
+        if constexpr (ES == 2)
+            if (a.rows0 == kTallRows)
+                return shape(mg_fine_kernel<MODE, FineSten, T, kTallRows>, FineLayout<MODE, ES, 12, kTallRows>());
+        return shape(mg_fine_kernel<MODE, FineSten, T, kRows>, FineLayout<MODE, ES, 12, kRows>());
     }
 
     // Partials per sum: the CTAs of the kernels that leave them.
     void count_parts(Args& out) const
     {
-        auto n = [&](auto fn, int tiles, int smem, int threads) { return ctas(fn, tiles, smem, threads); };
+        auto n = [&](auto fn, int tiles, int smem, int threads, int) { return ctas(fn, tiles, smem, threads); };
         out.n_pq = with_fine<FM_SPMV>(0, n);
         out.n_rz = with_fine<FM_UP>(0, n);
         out.n_rr = ctas(mg_update_kernel<false>, pointwise_tiles(), 0, kThreads);
@@ -2194,6 +2216,7 @@ int run_mg_solver(const gm_levin_store* store, const float* b, int bpitch, const
     a.alpha_out = alpha_out;
     a.rtol = p->rtol;
     a.outer_low = outer_low_for(tcode, a.rtol);
+    a.rows0 = level0_rows(a.W, a.H, sms);
     a.max_iters = p->max_iters;
     a.replace_every = p->replace_every;
     a.omega = p->mg_omega > 0.f ? p->mg_omega : kDefaultOmega;
@@ -2311,6 +2334,7 @@ extern "C" int gm_levin_solve_mg_many(const gm_levin_store* const* stores, float
         a.alpha_out = alphas[k];
         a.rtol = p.rtol;
         a.outer_low = outer_low_for(tcode, a.rtol);
+        a.rows0 = level0_rows(a.W, a.H, sms);
         a.max_iters = p.max_iters;
         a.replace_every = p.replace_every;
         a.omega = p.mg_omega > 0.f ? p.mg_omega : kDefaultOmega;
@@ -2408,6 +2432,7 @@ extern "C" int gm_levin_mg_inspect(const gm_levin_store* store, int use_low, con
     a.omega = kDefaultOmega;
     a.scale = kDefaultScale;
     a.max_iters = 1;
+    a.rows0 = level0_rows(a.W, a.H, sms);
     FineMaps fm;
     GM_TRY(make_maps(a, tcode ? 2 : 4, tcode_dtype(tcode), fm));
     cudaStream_t st = (cudaStream_t)stream;

@@ -67,13 +67,14 @@ def test_vcycle_matches_oracle(orc, prec):
 
 
 @pytest.mark.parametrize("W,H", [(16, 15), (17, 16), (23, 3), (72, 72), (73, 72), (145, 37), (80, 131), (300, 17),
-                                 (171, 131), (402, 283), (1300, 21)])
+                                 (171, 131), (402, 283), (1300, 21),
+                                 (1160, 520), (1290, 545)])
 def test_vcycle_dense_level_shapes(orc, W, H):
-    """Sizes around the limits of the dense level and of the two-level kernels: the
-    coarsest level alone, levels of
-    just under and just over the cell limit, one pair of levels, a pair below a
-    single level, odd sides and thin images.  Tolerance: the parity
-    bar of the FP32 V-cycle (1e-4)."""
+    """Sizes around the limits of the dense level, of the two-level kernels and of
+    the level-0 tile heights: the coarsest level alone, levels of just under and
+    just over the cell limit, one pair of levels, a pair below a single level,
+    short tiles with one and with two ring stages, tall tiles, odd sides and
+    thin images.  Tolerance: the parity bar of the FP32 V-cycle (1e-4)."""
     torch = torch_cuda()
     st, p, w, g, b = _store(orc, W, H, "fp16", seed=4)
     M, lv = _oracle_levels(st, g, "fp16")
