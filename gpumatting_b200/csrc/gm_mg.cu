@@ -1559,10 +1559,28 @@ static size_t carve(const Plan& pl, int P0, char* base, Args* a)
 // an execution stream (for batches), pinned state for the read-back, timing
 // events and a cache of instantiated graphs.  Single solves use slot 0;
 // gm_levin_solve_mg_many spreads its images over the slots.
+//
+// A graph serves any buffers of its shape and parameters: the kernels that use
+// a store's planes or the caller's vectors (the set-up, the replacement, the
+// level-0 passes and the final write, about 35 of 120 nodes) are given new ones
+// before a launch (10-25 us; a capture and instantiation takes 1-2 ms).
+enum { B_INIT = 0, B_BUILD0 = 1, B_REPLACE = 2, B_FINAL = 3, B_FINE = 4 };  // B_FINE + FM_*
+struct BoundNode {
+    cudaGraphNode_t node;
+    void* fn;
+    unsigned grid, threads, smem;
+    int kind, nst, pending;
+    unsigned long long cond, cond_outer;
+};
 struct Graph {
-    Args key;
+    Args key;             // the solve it is bound to
+    Args shape;           // the same without the fields a binding sets
+    Args launch;          // as captured (with the partial-sum counts)
     int tcode;
+    cudaGraph_t graph;    // owns the nodes
     cudaGraphExec_t exec;
+    std::vector<BoundNode> nodes;
+    int rebinds;
     unsigned long long used;
 };
 
@@ -1595,9 +1613,15 @@ static bool graph_enabled()
 static std::mutex g_mu;
 static Dev g_dev[64][kSlots];
 
+static void free_graph(Graph& g)
+{
+    cudaGraphExecDestroy(g.exec);
+    cudaGraphDestroy(g.graph);
+}
+
 static void drop_graphs(Dev& d)
 {
-    for (Graph& g : d.graphs) cudaGraphExecDestroy(g.exec);
+    for (Graph& g : d.graphs) free_graph(g);
     d.graphs.clear();
 }
 
@@ -1745,6 +1769,28 @@ struct Enq {
     cudaStream_t s;
     bool dry;
     const FineMaps* fm;
+    std::vector<BoundNode>* rec = nullptr;  // capture only: the nodes a binding sets
+
+    // Notes the kernel node captured last.
+    template <class K> void note(K fn, int tiles, int smem, int threads, int kind, int nst = 0, int pending = 0) const
+    {
+        if (!rec || dry) return;
+        cudaStreamCaptureStatus cs;
+        const cudaGraphNode_t* deps = nullptr;
+        size_t nd = 0;
+        BoundNode b = {};
+        if (cudaStreamGetCaptureInfo(s, &cs, nullptr, nullptr, &deps, &nd) == cudaSuccess && nd == 1) b.node = deps[0];
+        b.fn = (void*)fn;
+        b.grid = (unsigned)ctas(fn, tiles, smem, threads);
+        b.threads = (unsigned)threads;
+        b.smem = (unsigned)smem;
+        b.kind = kind;
+        b.nst = nst;
+        b.pending = pending;
+        b.cond = a.cond;
+        b.cond_outer = a.cond_outer;
+        rec->push_back(b);
+    }
 
     template <class K> int ctas(K fn, int tiles, int smem, int threads) const
     {
@@ -1781,6 +1827,7 @@ struct Enq {
         const TMaps& m = MODE == FM_SPMV ? fm->spmv : (MODE == FM_DOWN ? fm->down[l] : fm->up[l]);
         with_fine<MODE>(l, [&](auto fn, int tiles, int smem, int threads, int nst) {
             go(fn, tiles, smem, threads, m, a, l, nst, pending);
+            if (l == 0) note(fn, tiles, smem, threads, B_FINE + MODE, nst, pending);
         });
     }
 
@@ -1855,13 +1902,16 @@ struct Enq {
         constexpr int sm = (int)(sizeof(float) * FineSten::NP * (kTY + kHalo) * kPW +
                                  sizeof(double) * (kTY + 2 * kHalo) * kVW);
         go(mg_replace_kernel, tiles_of(a.W, a.H, kTY), sm, kThreads, a);
+        note(mg_replace_kernel, tiles_of(a.W, a.H, kTY), sm, kThreads, B_REPLACE);
     }
 
     void setup() const
     {
         go(mg_init_kernel, pointwise_tiles(), 0, kThreads, a);
+        note(mg_init_kernel, pointwise_tiles(), 0, kThreads, B_INIT);
         constexpr int sm0 = (int)sizeof(T) * FineSten::NP * (kBuildTY + kHalo) * kPW;
         go(mg_build0_kernel<T>, tiles_of(a.W, a.H, kBuildTY), sm0, kThreads, a);
+        note(mg_build0_kernel<T>, tiles_of(a.W, a.H, kBuildTY), sm0, kThreads, B_BUILD0);
         int l = 1;
         for (; l < a.L && (long long)a.lev[l + 1].W * a.lev[l + 1].H > kOneCtaCells; ++l)
             go(mg_build_kernel, (a.lev[l + 1].W * a.lev[l + 1].H + 127) / 128, 0, 128, a, l);
@@ -1888,7 +1938,11 @@ struct Enq {
         }
     }
 
-    void finish() const { go(mg_final_kernel, pointwise_tiles(), 0, kThreads, a); }
+    void finish() const
+    {
+        go(mg_final_kernel, pointwise_tiles(), 0, kThreads, a);
+        note(mg_final_kernel, pointwise_tiles(), 0, kThreads, B_FINAL);
+    }
 };
 
 // Iterations per pass of the inner loop.  Going round a WHILE node costs 3-6 us
@@ -1938,7 +1992,7 @@ static cudaError_t add_while(cudaStream_t s, cudaGraphConditionalHandle* h, cuda
 // The replacement kernel keeps or ends both loops, the update kernel ends the
 // inner one when a replacement is due.
 template <class T>
-static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec)
+static int build_graph(Dev& d, Args a, const FineMaps& fm, Graph& out)
 {
     cudaGraph_t g = nullptr, outer = nullptr, inner = nullptr;
     a.cond = a.cond_outer = 0;
@@ -1950,8 +2004,9 @@ static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec
         dry.count_parts(a);
         dry.finish();
     }
+    out.launch = a;
     GM_CUDA_TRY(cudaStreamBeginCapture(d.cap, cudaStreamCaptureModeThreadLocal));
-    Enq<T>{a, d.sms, d.cap, false, &fm}.setup();
+    Enq<T>{a, d.sms, d.cap, false, &fm, &out.nodes}.setup();
     cudaGraphConditionalHandle ho = 0, hi = 0;
     cudaError_t e = add_while(d.cap, &ho, &outer);
     if (e == cudaSuccess) {
@@ -1968,12 +2023,12 @@ static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec
             e = cudaStreamGetCaptureInfo(d.cap2, &cs, nullptr, &og, nullptr, nullptr);
             if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hi, og, 1, cudaGraphCondAssignDefault);
             ab.cond = (unsigned long long)hi;
-            if (e == cudaSuccess) Enq<T>{ab, d.sms, d.cap2, false, &fm}.replace();
+            if (e == cudaSuccess) Enq<T>{ab, d.sms, d.cap2, false, &fm, &out.nodes}.replace();
             if (e == cudaSuccess) e = add_while(d.cap2, &hi, &inner);
             if (e == cudaSuccess) {
                 e = cudaStreamBeginCaptureToGraph(d.cap3, inner, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
                 if (e == cudaSuccess) {
-                    const Enq<T> q{ab, d.sms, d.cap3, false, &fm};
+                    const Enq<T> q{ab, d.sms, d.cap3, false, &fm, &out.nodes};
                     q.iterations(unroll_for(a));
                     cudaGraph_t x = nullptr;
                     e = cudaStreamEndCapture(d.cap3, &x);
@@ -1984,12 +2039,13 @@ static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec
             if (e == cudaSuccess) e = e1;
         }
     }
-    if (e == cudaSuccess) Enq<T>{a, d.sms, d.cap, false, &fm}.finish();
+    if (e == cudaSuccess) Enq<T>{a, d.sms, d.cap, false, &fm, &out.nodes}.finish();
     cudaError_t e2 = cudaStreamEndCapture(d.cap, &g);
     if (e == cudaSuccess) e = e2;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
-    if (g) cudaGraphDestroy(g);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&out.exec, g, 0);
+    out.graph = g;
     if (e != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
         cudaGetLastError();
         gm_set_error_msg("multigrid graph capture: %s", cudaGetErrorString(e));
         return GM_ERR_CUDA;
@@ -1997,31 +2053,98 @@ static int build_graph(Dev& d, Args a, const FineMaps& fm, cudaGraphExec_t* exec
     return GM_OK;
 }
 
-// The cached graph of this solve on slot d, captured on first use.
+// The fields of a solve that a binding sets: copied from src, or cleared.
+static void bind_fields(Args& a, const Args* src)
+{
+    a.lev[0].c = src ? src->lev[0].c : nullptr;
+    a.lev[0].ps = src ? src->lev[0].ps : 0;
+    a.lev[0].D = src ? src->lev[0].D : nullptr;
+    a.w32 = src ? src->w32 : nullptr;
+    a.ps32 = src ? src->ps32 : 0;
+    a.gamma = src ? src->gamma : nullptr;
+    a.d32 = src ? src->d32 : nullptr;
+    a.bvec = src ? src->bvec : nullptr;
+    a.bpitch = src ? src->bpitch : 0;
+    a.alpha_in = src ? src->alpha_in : nullptr;
+    a.alpha_out = src ? src->alpha_out : nullptr;
+}
+
+// Gives the graph the buffers of solve a.  (Launches that are already enqueued
+// keep theirs.)
+static int rebind(Graph& g, const Args& a, const FineMaps& fm)
+{
+    Args b = g.launch;
+    bind_fields(b, &a);
+    for (const BoundNode& n : g.nodes) {
+        b.cond = n.cond;
+        b.cond_outer = n.cond_outer;
+        TMaps m;
+        int l = 0, nst = n.nst, pending = n.pending;
+        void* fine[] = {&m, &b, &l, &nst, &pending};
+        void* plain[] = {&b};
+        cudaKernelNodeParams kp = {};
+        kp.func = n.fn;
+        kp.gridDim = dim3(n.grid);
+        kp.blockDim = dim3(n.threads);
+        kp.sharedMemBytes = n.smem;
+        kp.kernelParams = plain;
+        if (n.kind >= B_FINE) {
+            const int mode = n.kind - B_FINE;
+            m = mode == FM_SPMV ? fm.spmv : (mode == FM_DOWN ? fm.down[0] : fm.up[0]);
+            kp.kernelParams = fine;
+        }
+        if (!n.node || cudaGraphExecKernelNodeSetParams(g.exec, n.node, &kp) != cudaSuccess) {
+            cudaGetLastError();
+            return GM_ERR_CUDA;
+        }
+    }
+    memcpy(&g.key, &a, sizeof(Args));
+    return GM_OK;
+}
+
+// The graph of solve a on slot d: one bound to it already, else one of its
+// shape, given its buffers, else a new one.  A program that goes round a few
+// sets of buffers gets a graph for each (up to kSameShape) once the bindings
+// have cost as much as a capture.  The reference is valid until the next call.
+constexpr int kSameShape = 4, kRebindsPerCapture = 50;
 template <class T>
 static int graph_for(Dev& d, const Args& a, const FineMaps& fm, int tcode, Graph** out)
 {
-    *out = nullptr;
-    for (Graph& g : d.graphs)
-        if (g.tcode == tcode && memcmp(&g.key, &a, sizeof(Args)) == 0) *out = &g;
-    if (*out) {
-        (*out)->used = ++d.clock;
+    Args shape;
+    memcpy(&shape, &a, sizeof(Args));
+    bind_fields(shape, nullptr);
+    Graph* old = nullptr;
+    int same = 0, rebinds = 0;
+    for (Graph& g : d.graphs) {
+        if (g.tcode != tcode || memcmp(&g.shape, &shape, sizeof(Args)) != 0) continue;
+        if (memcmp(&g.key, &a, sizeof(Args)) == 0) {
+            g.used = ++d.clock;
+            *out = &g;
+            return GM_OK;
+        }
+        ++same;
+        rebinds += g.rebinds;
+        if (!old || g.used < old->used) old = &g;
+    }
+    if (old && (same >= kSameShape || rebinds < same * kRebindsPerCapture) && rebind(*old, a, fm) == GM_OK) {
+        old->rebinds += 1;
+        old->used = ++d.clock;
+        *out = old;
         return GM_OK;
     }
-    cudaGraphExec_t ex = nullptr;
-    GM_TRY(build_graph<T>(d, a, fm, &ex));
-    if (d.graphs.size() >= (size_t)kGraphCache) {
-        auto old = std::min_element(d.graphs.begin(), d.graphs.end(),
-                                    [](const Graph& x, const Graph& y) { return x.used < y.used; });
-        cudaGraphExecDestroy(old->exec);
-        d.graphs.erase(old);
-    }
-    Graph g;
+    Graph g = {};
+    GM_TRY(build_graph<T>(d, a, fm, g));
     memcpy(&g.key, &a, sizeof(Args));
+    memcpy(&g.shape, &shape, sizeof(Args));
     g.tcode = tcode;
-    g.exec = ex;
     g.used = ++d.clock;
-    d.graphs.push_back(g);
+    if (d.graphs.size() >= (size_t)kGraphCache) {
+        auto lru = std::min_element(d.graphs.begin(), d.graphs.end(),
+                                    [](const Graph& x, const Graph& y) { return x.used < y.used; });
+        free_graph(*lru);
+        d.graphs.erase(lru);
+    }
+    d.graphs.push_back(std::move(g));
     *out = &d.graphs.back();
     return GM_OK;
 }
@@ -2032,35 +2155,16 @@ static int run(Dev& d, const Args& a0, const FineMaps& fm, int tcode, cudaStream
     Args a = a0;
     if (d.cond_ok != 0 && graph_enabled()) {
         Graph* hit = nullptr;
-        for (Graph& g : d.graphs)
-            if (g.tcode == tcode && memcmp(&g.key, &a, sizeof(Args)) == 0) hit = &g;
-        if (!hit) {
-            cudaGraphExec_t ex = nullptr;
-            const int rc = build_graph<T>(d, a, fm, &ex);
-            if (rc == GM_OK) {
-                if (d.graphs.size() >= (size_t)kGraphCache) {
-                    auto old = std::min_element(d.graphs.begin(), d.graphs.end(),
-                                                [](const Graph& x, const Graph& y) { return x.used < y.used; });
-                    cudaGraphExecDestroy(old->exec);
-                    d.graphs.erase(old);
-                }
-                Graph g;
-                memcpy(&g.key, &a, sizeof(Args));
-                g.tcode = tcode;
-                g.exec = ex;
-                g.used = 0;
-                d.graphs.push_back(g);
-                hit = &d.graphs.back();
-                d.cond_ok = 1;
-            } else if (d.cond_ok == -1) {
-                d.cond_ok = 0;  // conditional nodes unavailable: host-driven loop from now on
-                if (getenv("GM_MG_DEBUG")) fprintf(stderr, "gm_mg: graph path unavailable (%s)\n", gm_last_error());
-            } else {
-                return rc;
-            }
+        const int rc = graph_for<T>(d, a, fm, tcode, &hit);
+        if (rc == GM_OK) {
+            d.cond_ok = 1;
+        } else if (d.cond_ok == -1) {
+            d.cond_ok = 0;  // conditional nodes unavailable: host-driven loop from now on
+            if (getenv("GM_MG_DEBUG")) fprintf(stderr, "gm_mg: graph path unavailable (%s)\n", gm_last_error());
+        } else {
+            return rc;
         }
         if (hit) {
-            hit->used = ++d.clock;
             GM_CUDA_TRY(cudaEventRecord(d.e0, st));
             GM_CUDA_TRY(cudaGraphLaunch(hit->exec, st));
             GM_CUDA_TRY(cudaEventRecord(d.e1, st));
@@ -2113,11 +2217,9 @@ static int run_many(Dev* slots, int K, std::vector<Item>& items, int tcode, cuda
 {
     const int n = (int)items.size();
     Dev& d0 = slots[0];
-    std::vector<cudaGraphExec_t> ex(n);
-    for (int k = 0; k < n; ++k) {
+    for (int k = 0; k < n; ++k) {  // captures come before the timing
         Graph* g = nullptr;
         GM_TRY(graph_for<T>(slots[items[k].slot], items[k].a, items[k].fm, tcode, &g));
-        ex[k] = g->exec;
     }
     if (d0.pin_n < n) {
         if (d0.pin) cudaFreeHost(d0.pin);
@@ -2130,7 +2232,9 @@ static int run_many(Dev* slots, int K, std::vector<Item>& items, int tcode, cuda
     for (int j = 0; j < K; ++j) GM_CUDA_TRY(cudaStreamWaitEvent(slots[j].run, d0.e0, 0));
     for (int k = 0; k < n; ++k) {
         Dev& d = slots[items[k].slot];
-        GM_CUDA_TRY(cudaGraphLaunch(ex[k], d.run));
+        Graph* g = nullptr;
+        GM_TRY(graph_for<T>(d, items[k].a, items[k].fm, tcode, &g));
+        GM_CUDA_TRY(cudaGraphLaunch(g->exec, d.run));
         GM_CUDA_TRY(cudaMemcpyAsync(d0.pin + k, items[k].a.st, sizeof(State), cudaMemcpyDeviceToHost, d.run));
     }
     for (int j = 0; j < K; ++j) {

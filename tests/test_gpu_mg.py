@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from gpu_util import edge_image, oracle_problem, torch_cuda
+from gpumatting_b200.synth import make_problem
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-4
@@ -382,6 +383,43 @@ def test_mg_replacement_periods(orc, monkeypatch, every, count):
         assert res.status == 0 and res.iters == count and res.replacements == 1 + due
         outs.append(alpha.cpu().numpy())
     assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32))
+
+
+def test_mg_graph_serves_other_buffers(orc):
+    """A captured solve is given the buffers of the next one of its shape: stores
+    of one size (one a view into a batch canvas, with another plane stride),
+    several alphas and a right-hand side of its own, often enough for more than
+    one graph of the shape, each bit for bit as on its first solve."""
+    import ctypes as C
+
+    torch = torch_cuda()
+    from gpumatting_b200 import _lib as L
+    from gpumatting_b200 import api
+
+    W, H = 70, 41
+    a, b = (_store(orc, W, H, "fp16", seed=k)[0] for k in (1, 2))
+    bt = api.LevinBatch([(50, 30), (W, H)], "fp16")
+    p = make_problem(W, H, 3)
+    bt.assemble(1, torch.from_numpy(p.image).cuda(), torch.from_numpy(p.scribbles).cuda(), eps=p.eps)
+    view = bt.store_view(1)
+    rhs = torch.rand((H, W), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    prm = L.default_params(solver=L.GM_SOLVER_MG, rtol=0.0, max_iters=7)
+
+    def solve(kind, x):
+        x.fill_(0.25)
+        info = L.GmSolveInfo()
+        st = C.byref(view if kind == 2 else (b.s if kind == 1 else a.s))
+        if kind == 3:
+            L.check(L.load().gm_levin_solve_rhs(st, rhs.data_ptr(), x.data_ptr(), C.byref(prm), C.byref(info), 0))
+        else:
+            L.check(L.load().gm_levin_solve(st, x.data_ptr(), C.byref(prm), C.byref(info), 0))
+        return x
+
+    bufs = [torch.empty((H, W), device="cuda") for _ in range(5)]
+    first = [solve(k, bufs[0]).clone() for k in range(4)]
+    assert not torch.equal(first[0], first[1])
+    for i in range(260):
+        assert torch.equal(solve(i % 4, bufs[i % 5]), first[i % 4]), i
 
 
 def test_batch_solve_with_mg(orc):
