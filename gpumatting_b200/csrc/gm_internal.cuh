@@ -138,6 +138,34 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
+// L2 policy of the plane loads.  The planes of an operator are read once or
+// twice per iteration, the vectors by every kernel: where the vectors fit L2
+// but vectors and planes together do not, the planes' lines are marked to
+// leave first.  Us per iteration without and with: fused CG, FP32 store, 1080p
+// 35.5 / 31.6, FP16 28.2 / 28.0; multigrid with the FP32 outer product 1501 x 703
+// 61 / 58, 1080p 93.0 / 91.0.  Where the vectors do not fit either, the marked
+// lines only lose what reuse there was (4096^2: multigrid 474 / 491, a CG
+// replacement 2x slower), and smaller problems fit whole.
+constexpr long long kPlanesFirstMaxPixels = 3500000;  // 32 B of vectors per pixel against 126 MB of L2
+inline int planes_leave_first(long long pixels) { return pixels <= kPlanesFirstMaxPixels ? 1 : 0; }
+__device__ __forceinline__ uint64_t plane_policy(int leave_first)
+{
+    uint64_t p;
+    if (leave_first) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
+__device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar,
+                                                 uint64_t policy)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+        " [%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)), "l"(policy)
+        : "memory");
+}
+
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");

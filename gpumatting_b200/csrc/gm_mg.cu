@@ -137,7 +137,8 @@ struct Args {
     float* xinc;          // FP32 increment since the last replacement [H][P]
     float *r, *q, *p0, *p1;  // fine vectors [H][P]; z is lev[0].x
     double* parts;        // [5][kMaxParts], S_*
-    int n_pq, n_rr, n_rz, spare0; // partials per sum: the CTAs of the kernel that leaves them
+    int planes_first;     // plane_policy of the level-0 planes
+    int n_pq, n_rr, n_rz; // partials per sum: the CTAs of the kernel that leaves them
     State* st;
     double rtol;
     int max_iters, replace_every;
@@ -787,7 +788,10 @@ __global__ void __launch_bounds__(32 * ROWS, 1)
     __syncthreads();
     auto issue_planes = [&](int t, int s) {
         const int u0 = (t % ntx) * kFTW, v0 = (t / ntx) * TH;
-        tma_load_3d(smem + s * LY::stage, &tm.m[0], u0 - 8, v0 - 2, 0, &full[s]);
+        if (S::NP == 12)
+            tma_load_3d_hint(smem + s * LY::stage, &tm.m[0], u0 - 8, v0 - 2, 0, &full[s], plane_policy(a.planes_first));
+        else
+            tma_load_3d(smem + s * LY::stage, &tm.m[0], u0 - 8, v0 - 2, 0, &full[s]);
     };
     // The planes are constant during a solve (written by the store's assembly
     // or the set-up kernels, which completed before this kernel's predecessor
@@ -2321,6 +2325,7 @@ int run_mg_solver(const gm_levin_store* store, const float* b, int bpitch, const
     a.rtol = p->rtol;
     a.outer_low = outer_low_for(tcode, a.rtol);
     a.rows0 = level0_rows(a.W, a.H, sms);
+    a.planes_first = planes_leave_first((long long)a.W * a.H);
     a.max_iters = p->max_iters;
     a.replace_every = p->replace_every;
     a.omega = p->mg_omega > 0.f ? p->mg_omega : kDefaultOmega;
@@ -2439,6 +2444,7 @@ extern "C" int gm_levin_solve_mg_many(const gm_levin_store* const* stores, float
         a.rtol = p.rtol;
         a.outer_low = outer_low_for(tcode, a.rtol);
         a.rows0 = level0_rows(a.W, a.H, sms);
+        a.planes_first = planes_leave_first((long long)a.W * a.H);
         a.max_iters = p.max_iters;
         a.replace_every = p.replace_every;
         a.omega = p.mg_omega > 0.f ? p.mg_omega : kDefaultOmega;
@@ -2537,6 +2543,7 @@ extern "C" int gm_levin_mg_inspect(const gm_levin_store* store, int use_low, con
     a.scale = kDefaultScale;
     a.max_iters = 1;
     a.rows0 = level0_rows(a.W, a.H, sms);
+    a.planes_first = planes_leave_first((long long)a.W * a.H);
     FineMaps fm;
     GM_TRY(make_maps(a, tcode ? 2 : 4, tcode_dtype(tcode), fm));
     cudaStream_t st = (cudaStream_t)stream;

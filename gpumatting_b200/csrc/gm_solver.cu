@@ -295,6 +295,7 @@ __device__ __forceinline__ void run_sweep(const SolverArgs& A, const UnitGeo& ge
         const CUtensorMap* xm = KIND == KIND_KRYLOV ? &A.m_xlo : &A.m_xhi;
         const uint32_t vbytes = K.vbytes[0] + K.vbytes[1] + K.vbytes[2] + K.vbytes[3] + (vm[4] ? K.vbytes[4] : 0);
         fence_proxy_async();
+        const uint64_t policy = plane_policy(A.planes_first);
         // Issue in the consumers' order: super-step j takes vector rows j and
         // j+1, then band rows up to (its last step) - 2.  Matching the order
         // keeps the rings deadlock-free for any depth >= 1.
@@ -324,7 +325,7 @@ __device__ __forceinline__ void run_sweep(const SolverArgs& A, const UnitGeo& ge
             pp.used_b |= bit;
             unsigned char* dst = bring + bs * K.bslot;
             mbar_arrive_expect_tx(&full[kRvMax + bs], K.bbytes);
-            tma_load_3d(dst, bm, u0 - 8, v0 - 2 + m, 0, &full[kRvMax + bs]);
+            tma_load_3d_hint(dst, bm, u0 - 8, v0 - 2 + m, 0, &full[kRvMax + bs], policy);
             if (K.xoff >= 0) tma_load_2d(dst + K.xoff, xm, u0 - 8, v0 - 2 + m, &full[kRvMax + bs]);
             bs = ring_next(bs, K.Rb);
             return true;

@@ -226,6 +226,7 @@ struct SolverArgs {
     float omega;
     uint64_t limit_ns;       // grid-barrier wait limit
     uint64_t tma_limit_ns;   // TMA / ring wait limit (never below 2 s)
+    int planes_first;        // plane_policy of the band rows
     int inject;              // 1: first grid barrier expects one extra arrival
     // batched solves (BATCH kernels only)
     const BatchImage* imgs;
