@@ -128,30 +128,34 @@ struct SymOut {
 // (3 - |du| windows per pair) take 9 values per row through shared memory.
 // The thread of column u finishes the couplings with du = -1, 0, 1 of pixel u,
 // du = 2 of pixel u - 1 and du = -2 of pixel u + 1 (one window column only).
-// The rounded couplings go through a ring in shared memory, from which the
-// diagonal (the sum of exactly the stored weights) is formed in the same pass
-// instead of in a second one that reads all planes again (84 B/px).  The first
+// The diagonal (the FP64 sum of exactly the stored weights) is formed in the same
+// pass instead of in a second one that reads all planes again (84 B/px): the
+// thread that finishes a coupling adds it to the sums of both its pixels, which
+// lie in its own column or a neighbouring one, in this row or the two below, and
+// hands the neighbours' sums over once per row.  The first
 // rows of a run repeat the couplings of the two rows above it; runs are as
 // long as one wave of CTAs allows.
 //
-// Measured with the FP16 store: 1080p RGB8 450 -> 122 us, 4096^2 870 us (83 B
-// written per pixel are 26 and 215 us); FP32 store, 4001 x 2999: 2,400 -> 540
-// (RGB8), 620 us (float).  Bound by instruction issue at 12 warps per SM (59 %
-// of the slots, FP64 pipe 37 %); a first form that kept the windows in shared
-// memory took 156 us, bound by its reads (12 shared wavefronts per 32 pixels
-// and window).
+// Measured with the FP16 store: 1080p RGB8 450 -> 117 us, 4096^2 850 us (83 B
+// written per pixel are 26 and 215 us); FP32 store, 4001 x 2999: 2,400 -> 500
+// (RGB8), 560 us (float).  Bound by instruction issue at 12 warps per SM (about 60
+// % of the slots, FP64 pipe 37 %).  Forms before: windows in shared memory 156 us
+// (12 shared wavefronts per 32 pixels and window); all rounded couplings through a
+// shared ring for the diagonal 122.
 constexpr int kAT = 128;              // threads = window columns
 constexpr int kAW = kAT - 2;          // output columns per CTA
 constexpr int kAP = kAT + 4;          // row length in shared memory (two pad columns each side)
 // CTAs per SM the registers are cut for.  A float image's 27 colours and 18 row
 // sums in 64 bits spill at 168 registers (1080p: 160 us with 3 CTAs per SM, 135
-// with 2); an RGB8 image's do not (122 us with 3, 135 with 2).
+// with 2); an RGB8 image's do not (122 us with 3, 135 with 2; before the diagonal
+// moved to registers).
 __host__ __device__ constexpr int asm_ctas(bool f32) { return f32 ? 2 : 3; }
 constexpr int kMinRows = 2;
 
-// Rows of the coupling ring: couplings to the same row are read in the step
-// that forms them, those to the next row one step later, to the second row
-// two steps later.
+// Rows of the coupling rings (the 25-band output, whose lower bands repeat the
+// couplings of rows above, and the low-precision weights of float images): couplings to the same row are read in the step that
+// forms them, those to the next row one step later, to the second row two
+// steps later.
 __host__ __device__ constexpr int ring_base(int k) { return k <= 2 ? k - 1 : (k <= 7 ? 2 + 2 * (k - 3) : 12 + 3 * (k - 8)); }
 __host__ __device__ constexpr int ring_len(int k) { return k <= 2 ? 1 : (k <= 7 ? 2 : 3); }
 constexpr int kRingRows = 27;
@@ -168,18 +172,24 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
                                                                        int rows, SymOut o)
 {
     constexpr bool kLow = sizeof(T) == 2;
+    // Two sets of nine FP64 sums do not fit beside a float image's registers
+    // (1080p: 148 us against 130): there the low-precision weights go through a
+    // ring in shared memory and are summed from it.
+    constexpr bool kLowRing = kLow && F32IMG;
     using Sum = typename std::conditional<F32IMG, double, int>::type;
     using Pix = typename std::conditional<F32IMG, float, int>::type;
     __shared__ double xch[9][kAP];
-    __shared__ float hi[kRingRows][kAP];
-    __shared__ T lo[kLow ? kRingRows : 1][kAP];
+    __shared__ double sums[kLow && !kLowRing ? 4 : 2][kAP];  // this row's shares of the left and right columns' diagonals
+    __shared__ float hi[BANDS ? kRingRows : 1][kAP];
+    __shared__ T lo[kLowRing ? kRingRows : 1][kAP];
     const int t = threadIdx.x, c = t + 2, u = blockIdx.x * kAW - 1 + t;
     const int r0 = blockIdx.y * rows, r1 = min(r0 + rows, H), rs0 = max(r0 - 2, 0);
     const bool ok_col = u >= 1 && u <= W - 2;
-    for (int i = t; i < kRingRows * kAP; i += kAT) {
-        hi[i / kAP][i % kAP] = 0.f;
-        if (kLow) lo[i / kAP][i % kAP] = T(0.f);
-    }
+    if (BANDS || kLowRing)
+        for (int i = t; i < kRingRows * kAP; i += kAT) {
+            if (BANDS) hi[i / kAP][i % kAP] = 0.f;
+            if (kLowRing) lo[i / kAP][i % kAP] = T(0.f);
+        }
 
     // Colours (u - 1, u, u + 1) of row v, zero outside the image (and in an
     // image without any window, whatever its colours hold).
@@ -229,6 +239,9 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
     for (int n = 0; n < 9; ++n) dn1[n] = 0.0;
 #pragma unroll
     for (int n = 0; n < 3; ++n) in0[n] = in1[n] = 0.0;
+    // Diagonal sums of rows r, r + 1, r + 2 in the columns left of, at and right of
+    // this thread's: of the FP32 weights, and of the low-precision ones.
+    double d32[3][3] = {}, dlo[3][3] = {};
     const size_t plane = o.plane;
     T* wl = reinterpret_cast<T*>(o.w);
     const bool own_w = o.w != (void*)o.w32;  // an FP32 store may keep w apart from w32
@@ -349,23 +362,31 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
         if (r < rs0) continue;
         __syncthreads();
         // --- finish the couplings of row r
-        double su = 0.0, su32 = 0.0;  // this pixel's own upper couplings, as rounded
         const int r2 = r & 1, r3 = r % 3;
         const bool row_out = r >= r0 && o.w32 != nullptr;
         const bool st[3] = {row_out && u > first && u <= last + 1, row_out && out_col, row_out && u >= first - 1 && u < last};
         float* w32 = o.w32 + (size_t)r * o.pitch + u;
         T* wlo = wl + (size_t)r * o.pitch + u;
-        auto finish = [&](int k, int x, double w9) {  // x: pixel column less u
+        // x: column of the upper pixel less u; the lower one is du further, dv below
+        auto finish = [&](int k, int x, double w9) {
+            const int dv = (k + 2) / 5, du = k - 5 * dv;
             const double w = w9 * (1.0 / 9.0);
             const float wf = __double2float_rn(w);
-            const int row = ring_base(k) + (ring_len(k) == 1 ? 0 : (ring_len(k) == 2 ? r2 : r3));
-            hi[row][c + x] = wf;
-            if (x == 0) su32 += (double)wf;
+            const int row = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2 : r3));
+            if (BANDS) hi[row][c + x] = wf;
+            const double wd = (double)wf;
+            d32[0][1 + x] += wd;
+            d32[dv][1 + x + du] += wd;
             if (st[x + 1]) w32[(size_t)(k - 1) * plane + x] = wf;
             if (kLow) {
                 const T wt = from_double<T>(w);
-                lo[row][c + x] = wt;
-                if (x == 0) su += (double)Cvt<T>::to_f(wt);
+                if (kLowRing) {
+                    lo[row][c + x] = wt;
+                } else {
+                    const double wd2 = (double)Cvt<T>::to_f(wt);
+                    dlo[0][1 + x] += wd2;
+                    dlo[dv][1 + x + du] += wd2;
+                }
                 if (st[x + 1]) wlo[(size_t)(k - 1) * plane + x] = wt;
             } else if (own_w && st[x + 1]) {
                 wlo[(size_t)(k - 1) * plane + x] = from_double<T>(w);
@@ -383,34 +404,43 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
         finish(3, 1, p1[6]);
         finish(1, 0, p0[2] + xch[8][c + 1]);
         finish(2, -1, p0[1]);
+        sums[0][c] = d32[0][0];
+        sums[1][c] = d32[0][2];
+        if (kLow && !kLowRing) {
+            sums[2][c] = dlo[0][0];
+            sums[3][c] = dlo[0][2];
+        }
+        const double own32 = d32[0][1], own = dlo[0][1];
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            d32[0][n] = d32[1][n]; d32[1][n] = d32[2][n]; d32[2][n] = 0.0;
+            dlo[0][n] = dlo[1][n]; dlo[1][n] = dlo[2][n]; dlo[2][n] = 0.0;
+        }
         __syncthreads();
-        // --- diagonal of row r from the rounded couplings
+        // --- diagonal of row r
         if (out) {
             const size_t gi = (size_t)r * o.pitch + u;
             // Matting.cu:205-216: 255 -> (gamma, b = gamma), 0 -> (gamma, b = 0)
             const bool mark = sc_m == 255 || sc_m == 0;
             const float gam = sc.gamma_map ? sc_g : (mark ? sc.gamma_value : 0.f);
             const float bv = sc.gamma_map ? (sc.s_map ? sc_g * sc_s : 0.f) : (sc_m == 255 ? sc.gamma_value : 0.f);
-            double s1 = (double)gam + su, s32 = (double)gam + su32;
             const int r2b = r2 ^ 1, r3b = r3 == 2 ? 0 : r3 + 1;  // rows r - 1 (mod 2), r - 2 (mod 3)
-            float below[13];
+            double s1 = 0.0;
+            if (kLowRing) {
 #pragma unroll
-            for (int k = 1; k <= 12; ++k) {
-                const int dv = (k + 2) / 5, du = k - 5 * dv;
-                const int up = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2 : r3));
-                const int dn = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2b : r3b));
-                if (du == 2 || du == -2) s32 += (double)hi[up][c];
-                s32 += (double)hi[dn][c - du];
-                if (kLow) {
-                    if (du == 2 || du == -2) s1 += (double)Cvt<T>::to_f(lo[up][c]);
-                    s1 += (double)Cvt<T>::to_f(lo[dn][c - du]);
+                for (int k = 1; k <= 12; ++k) {
+                    const int dv = (k + 2) / 5, du = k - 5 * dv;
+                    s1 += (double)Cvt<T>::to_f(lo[ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2 : r3))][c]);
+                    s1 += (double)Cvt<T>::to_f(lo[ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2b : r3b))][c - du]);
                 }
-                if (BANDS) below[k] = hi[dn][c - du];
+            } else if (kLow) {
+                s1 = own + (sums[2][c + 1] + sums[3][c - 1]);
             }
+            const double s32 = (double)gam + (own32 + (sums[0][c + 1] + sums[1][c - 1]));
             if (o.d32) {
                 o.gamma[gi] = gam;
                 o.b[gi] = bv;
-                o.d[gi] = __double2float_rn(kLow ? s1 : s32);
+                o.d[gi] = __double2float_rn(kLow ? (double)gam + s1 : s32);
                 o.d32[gi] = __double2float_rn(s32);
             }
             if (BANDS) {
@@ -419,9 +449,9 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
 #pragma unroll
                 for (int k = -12; k <= 12; ++k) {
                     if (k == 0) continue;
-                    const int ka = k < 0 ? -k : k;
-                    const int up = ring_base(ka) + (ring_len(ka) == 1 ? 0 : (ring_len(ka) == 2 ? r2 : r3));
-                    const float a = -(k < 0 ? below[ka] : hi[up][c]);
+                    const int ka = k < 0 ? -k : k, dv = (ka + 2) / 5, du = ka - 5 * dv;
+                    const int row = ring_base(ka) + (dv == 0 ? 0 : (dv == 1 ? (k < 0 ? r2b : r2) : (k < 0 ? r3b : r3)));
+                    const float a = -(k < 0 ? hi[row][c - du] : hi[row][c]);
                     o.a25[(size_t)(12 + k) * o.apitch + i] = a;
                     rs -= (double)a;
                 }
