@@ -112,13 +112,16 @@ cudaError_t gm_scratch_alloc(void** p, size_t bytes, cudaStream_t st)
 
 // Stores come and go with the images of a training loop, and the driver's
 // cudaMalloc and cudaFree of one take 0.4-0.6 ms each (spikes of 10-20 ms were
-// seen): stores of up to 256 MiB come from a pool that keeps as much mapped and
-// gives back what exceeds it.  The memory is ready for any stream on return.
-constexpr size_t kStorePoolBytes = 256ull << 20;
+// seen): stores of up to 64 MiB (0.7 Mpixel in FP16) come from a pool that keeps
+// up to 512 MiB mapped and gives back what exceeds it.  Larger ones do not: a few
+// of them alive are past any such bound, and the pool then maps their memory
+// anew each time, which took 0.93 ms at 1080p against cudaMalloc's 0.43.  The
+// memory is ready for any stream on return.
+constexpr size_t kPooledStoreBytes = 64ull << 20, kStorePoolBytes = 512ull << 20;
 cudaError_t gm_store_malloc(void** p, size_t bytes)
 {
     static PoolCache cache;
-    if (bytes <= kStorePoolBytes) {
+    if (bytes <= kPooledStoreBytes) {
         const PoolCache::Entry e = library_pool(cache, kStorePoolBytes, true);
         if (e.pool && cudaMallocFromPoolAsync(p, bytes, e.pool, e.stream) == cudaSuccess)
             return cudaStreamSynchronize(e.stream);
