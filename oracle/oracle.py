@@ -30,7 +30,7 @@ def build(ref: bool | None = None) -> None:
     """Compile liborc.so and, when the reference tree is present, _ref."""
     subprocess.check_call(["make", "-s", "-C", HERE, "all"])
     if ref is None:
-        ref = os.path.isdir(REF_TREE)
+        ref = os.path.isfile(os.path.join(REF_TREE, "Matting.cu"))  # the directory alone may be empty
     if ref:
         subprocess.check_call(["make", "-s", "-C", HERE, "ref", f"REF={REF_TREE}"])
 
