@@ -142,8 +142,8 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 // twice per iteration, the vectors by every kernel: where the vectors fit L2
 // but vectors and planes together do not, the planes' lines are marked to
 // leave first.  Us per iteration without and with: fused CG, FP32 store, 1080p
-// 35.5 / 31.6, FP16 28.2 / 28.0; multigrid with the FP32 outer product 1501 x 703
-// 61 / 58, 1080p 93.0 / 91.0.  Where the vectors do not fit either, the marked
+// 35.8 / 31.7, FP16 28.5 / 28.3, within 0.5 % up to 1400 x 760; multigrid with the
+// FP32 outer product 1501 x 703 61 / 58, 1080p 93.0 / 91.0.  Where the vectors do not fit either, the marked
 // lines only lose what reuse there was (4096^2: multigrid 474 / 491, a CG
 // replacement 2x slower), and smaller problems fit whole.
 constexpr long long kPlanesFirstMaxPixels = 3500000;  // 32 B of vectors per pixel against 126 MB of L2

@@ -1,14 +1,14 @@
 // gm_levin.cu -- Levin matting Laplacian assembly on the GPU.
 //
-// Gather form (no atomics): a CTA covers a TW x TH pixel tile.  It stages
-// the tile's colours plus a 2-pixel halo, computes the statistics of every
-// 3x3 window touching the tile once (mean and regularised inverse
-// covariance), then each thread sums, for its own pixel i and each of the 24
-// neighbours j of the 5x5 stencil, the window terms
+// No atomics: every entry is written once, by one thread.  Per pixel i and
+// each of the 24 neighbours j of the 5x5 stencil, the window terms
 //     (1 + (x_i - mu)^T (Sigma + eps/9 I)^-1 (x_j - mu)) / 9
-// over the windows holding both, in window raster order (Matting.cu:79-189,
-// matlab/getLevinLapRaster.m:22-62).  Rows therefore need no cross-thread
-// reduction and every entry is written once.
+// are summed over the 3x3 windows holding both (Matting.cu:79-189,
+// matlab/getLevinLapRaster.m:22-62).  levin_sym_kernel goes by windows (one
+// thread per window column, marching down); levin_ref_kernel gathers: a CTA
+// stages a TW x TH pixel tile with a 2-pixel halo and the statistics of every
+// window that touches it, then each thread sums its pixel's rows in window
+// raster order.
 //
 // Two arithmetic modes:
 //   levin_sym_kernel   FP64 throughout, rounded once to the store types

@@ -27,15 +27,14 @@
 // (mg_dense_kernel).
 //
 // Outer loop: PCG with FP64 solution (plus an FP32 increment folded in after
-// each replacement), FP32 vectors and FP64 scalars on the true FP32 operator;
-// only the preconditioner reads the low-precision planes (the few MG
-// iterations make the outer operator's bytes minor, and a BF16 outer operator
-// would stall the recurrence).  The true residual b - A x in FP64 arithmetic
+// each replacement), FP32 vectors and FP64 scalars, on the FP16 planes where
+// outer_low_for allows it and else on the true FP32 operator; the
+// preconditioner reads the low-precision planes.  The true residual b - A x in FP64 arithmetic
 // replaces the recurrence every `replace_every` iterations and decides
 // convergence (the same reliable-update rule as the fused CG).
 // All scalars stay on the device: every reduction adds per-CTA partials in a
-// fixed order (so results are deterministic), in the kernel that needs it, and the whole
-// solve is ONE CUDA graph launch with two device-side conditional WHILE loops,
+// fixed order (so results are deterministic), p.q and r.z in the kernel that
+// needs them, and the whole solve is ONE CUDA graph launch with two device-side conditional WHILE loops,
 // over the residual replacements and, inside, over the iterations between
 // them -- no host round trip per iteration.  Kernels are
 // chained with programmatic dependent launch.  gm_levin_solve_mg_many runs
@@ -196,8 +195,10 @@ __device__ __forceinline__ void load_planes(T* sm, const T* g, size_t ps, int P,
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// Deterministic grid reductions: each CTA publishes its partial sums, the
-// last CTA to arrive adds all partials in index order.
+// Deterministic grid reductions: each CTA publishes its partial sums, and
+// either the last CTA to arrive adds them in index order (the sums that end a
+// recurrence) or every CTA of the consuming kernel does (p.q, r.z: no ticket,
+// and the sum is formed after a wait that the consumer makes anyway).
 // ---------------------------------------------------------------------------
 template <int NV>
 __device__ __forceinline__ bool last_cta_total(double (&v)[NV], double* parts, unsigned* ticket)
@@ -659,15 +660,16 @@ __global__ void __launch_bounds__(kThreads) mg_dense_kernel(Args a)
 }
 
 // ---------------------------------------------------------------------------
-// Level-0 kernels: persistent CTAs streaming 128-column tiles through a
-// two-stage TMA ring (the pattern of the standalone SpMV).  One elected
+// The kernels of level 0 and of the large coarse levels: persistent CTAs
+// streaming 128-column tiles through a TMA ring of two stages (one where every
+// tile has a CTA of its own; the pattern of the standalone SpMV).  One elected
 // thread issues, per tile, a 3-D box {144, TH + 2, 12} of the affinity planes
 // (8 columns each side so the box starts on a 16-byte boundary, 2 rows above
 // for the mirrored couplings) and 2-D boxes {144, TH + 4} of the vectors the
 // stencil input is made of; TMA's zero fill stands in for everything outside
 // the image.  After a stage lands, the CTA forms the stencil input in a
-// shared tile, then each thread marches TH / 4 rows of a column pair with a
-// 5 x 6 window of it in registers.
+// shared tile, then each thread takes two rows of a column pair with a 5 x 6
+// window of it in registers.
 //   FM_SPMV  input z + beta p_old, beta from the prolongation's r . z;
 //            q = A p_new with the FP32 planes and d32 (FP16 planes and d when
 //            Args::outer_low); writes p_new and q, sums p_new . q.
@@ -795,7 +797,7 @@ __global__ void __launch_bounds__(32 * ROWS, 1)
     };
     // The planes are constant during a solve (written by the store's assembly
     // or the set-up kernels, which completed before this kernel's predecessor
-    // began), so the first two stages' plane boxes are requested before the
+    // began), so the first stages' plane boxes are requested before the
     // wait for the predecessor; the stage's arrival comes with the vectors.
     const int npre = (t0 < ntiles ? 1 : 0) + (nst > 1 && t0 + G < ntiles ? 1 : 0);
     if (tid == 0)
@@ -1516,7 +1518,8 @@ static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Workspace carve: fine vectors r, q, p0, p1, z (FP32) and x (FP64) with the
 // store's pitch; per coarse level 4 coupling planes, D, Gamma, b, x (FP32,
-// pitch a multiple of 32); the coarsest inverse; reduction partials; state.
+// pitch a multiple of 32); the matrices of the dense levels (FP64, 13.5 MB at
+// most for the largest); reduction partials; state.
 static size_t carve(const Plan& pl, int P0, char* base, Args* a)
 {
     size_t off = 0;
