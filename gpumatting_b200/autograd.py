@@ -12,7 +12,49 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib as L
 from . import api
+
+# Stores of up to this size (0.7 Mpixel in FP16) are tensors of torch's caching
+# allocator: a training loop makes one per step, and the driver's cudaMalloc and
+# cudaFree of one take 0.4-0.6 ms (spikes of 10-20 ms were seen) of a step's 6 at
+# 512x512.  That memory is ordered by the stream it was made on, which is right
+# here and not for api.LevinStore: the solves and the adjoint of one node run on
+# the stream that is current in its forward pass.  Next to the solves of a
+# larger image the allocation is small (under 2 % at 1080p), and its memory goes
+# back to the driver.
+CACHED_STORE_BYTES = 64 << 20
+
+
+class _CachedStore(api.LevinStore):
+    """api.LevinStore over memory of torch's caching allocator."""
+
+    def __init__(self, W: int, H: int, precision: str, memory):
+        P, esize = (W + 7) // 8 * 8, 4 if precision == "fp32" else 2
+        high, low, one = _plane_bytes(W, H, precision)
+        self.memory = memory
+        w32 = memory.data_ptr()
+        w = w32 if esize == 4 else w32 + high
+        gamma = w32 + high + low
+        self.s = L.GmLevinStore(W, H, P, api.PRECISIONS[precision], w, w32, gamma, gamma + one, gamma + 2 * one,
+                                gamma + 3 * one, 0, 0)
+        self.W, self.H, self.precision = W, H, precision
+
+
+def _plane_bytes(W: int, H: int, precision: str):
+    """Bytes of the 12 FP32 planes, of the 12 two-byte ones and of one vector, in
+    multiples of 256 as gm_levin_store_alloc lays them out."""
+    n = (W + 7) // 8 * 8 * H
+    return [(x + 255) // 256 * 256 for x in (48 * n, 0 if precision == "fp32" else 24 * n, 4 * n)]
+
+
+def _new_store(W: int, H: int, precision: str) -> api.LevinStore:
+    if W > 0 and H > 0 and precision in api.PRECISIONS:
+        high, low, one = _plane_bytes(W, H, precision)
+        size = high + low + 4 * one
+        if size <= CACHED_STORE_BYTES:
+            return _CachedStore(W, H, precision, torch.empty(size, dtype=torch.uint8, device="cuda"))
+    return api.LevinStore(W, H, precision)
 
 
 class LevinMatte(torch.autograd.Function):
@@ -28,7 +70,7 @@ class LevinMatte(torch.autograd.Function):
         im4[..., :3] = image.detach()
         g = gamma.detach().to(torch.float32).contiguous()
         sv = s.detach().to(torch.float32).contiguous()
-        store = api.LevinStore(W, H, precision).assemble(im4, gamma_map=g, s_map=sv, eps=eps)
+        store = _new_store(W, H, precision).assemble(im4, gamma_map=g, s_map=sv, eps=eps)
         alpha = torch.full((H, W), 0.5, dtype=torch.float32, device=image.device)
         res = store.solve(alpha, solver, rtol=rtol, max_iters=max_iters)
         ctx.store = store

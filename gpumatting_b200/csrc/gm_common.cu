@@ -63,79 +63,44 @@ unsigned long long gm_context_id()
 // per device and context, with a 64 MiB release threshold keeps these
 // buffers mapped.  Under stream capture, or when the context id is unknown,
 // the default pool is used.
-struct PoolCache {
-    struct Entry { unsigned long long ctx; cudaMemPool_t pool; cudaStream_t stream; };
-    static constexpr int kMaxDevices = 64;
-    std::mutex mu;
-    Entry entry[kMaxDevices] = {};
-};
-
-// The current device's entry of a cache of pools that keep up to `keep` bytes
-// mapped (with a stream of its own when asked for), or an empty one.
-static PoolCache::Entry library_pool(PoolCache& cache, uint64_t keep, bool with_stream)
+static cudaMemPool_t scratch_pool()
 {
+    constexpr int kMaxDevices = 64;
+    struct Entry { unsigned long long ctx; cudaMemPool_t pool; };
+    static std::mutex mu;
+    static Entry cache[kMaxDevices] = {};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= PoolCache::kMaxDevices) return {};
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
     const unsigned long long ctx = gm_context_id();
-    if (ctx == 0) return {};
-    std::lock_guard<std::mutex> lock(cache.mu);
-    PoolCache::Entry& e = cache.entry[dev];
-    if (e.pool && e.ctx == ctx) return e;
+    if (ctx == 0) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    Entry& e = cache[dev];
+    if (e.pool && e.ctx == ctx) return e.pool;
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    PoolCache::Entry n = {};
-    if (cudaMemPoolCreate(&n.pool, &props) != cudaSuccess ||
-        (with_stream && cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking) != cudaSuccess)) {
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
         cudaGetLastError();
-        return {};
+        return nullptr;
     }
-    cudaMemPoolSetAttribute(n.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    n.ctx = ctx;
-    e = n;
-    return e;
+    uint64_t keep = 64ull << 20;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    e.ctx = ctx;
+    e.pool = pool;
+    return pool;
 }
 
 cudaError_t gm_scratch_alloc(void** p, size_t bytes, cudaStream_t st)
 {
-    static PoolCache cache;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
     if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
-        const PoolCache::Entry e = library_pool(cache, 64ull << 20, false);
-        if (e.pool) return cudaMallocFromPoolAsync(p, bytes, e.pool, st);
+        if (cudaMemPool_t pool = scratch_pool()) return cudaMallocFromPoolAsync(p, bytes, pool, st);
     }
     cudaGetLastError();
     return cudaMallocAsync(p, bytes, st);
-}
-
-// Stores come and go with the images of a training loop, and the driver's
-// cudaMalloc and cudaFree of one take 0.4-0.6 ms each (spikes of 10-20 ms were
-// seen): stores of up to 64 MiB (0.7 Mpixel in FP16) come from a pool that keeps
-// up to 512 MiB mapped and gives back what exceeds it.  Larger ones do not: a few
-// of them alive are past any such bound, and the pool then maps their memory
-// anew each time, which took 0.93 ms at 1080p against cudaMalloc's 0.43.  The
-// memory is ready for any stream on return.
-constexpr size_t kPooledStoreBytes = 64ull << 20, kStorePoolBytes = 512ull << 20;
-cudaError_t gm_store_malloc(void** p, size_t bytes)
-{
-    static PoolCache cache;
-    if (bytes <= kPooledStoreBytes) {
-        const PoolCache::Entry e = library_pool(cache, kStorePoolBytes, true);
-        if (e.pool && cudaMallocFromPoolAsync(p, bytes, e.pool, e.stream) == cudaSuccess)
-            return cudaStreamSynchronize(e.stream);
-        cudaGetLastError();
-    }
-    return cudaMalloc(p, bytes);
-}
-
-// Freed memory of the pool may be handed out again at once, so every use of it
-// has to be over (cudaFree waits by itself only for memory of cudaMalloc).
-void gm_store_free(void* p)
-{
-    cudaDeviceSynchronize();
-    cudaFree(p);
 }
 
 int gm_check_device(int* sm_count)

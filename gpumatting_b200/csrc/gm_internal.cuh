@@ -46,11 +46,6 @@ unsigned long long gm_context_id();
 // synchronisations (free with cudaFreeAsync).
 cudaError_t gm_scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 
-// Device memory of a store, usable on any stream.  gm_store_free waits for the
-// device.
-cudaError_t gm_store_malloc(void** p, size_t bytes);
-void gm_store_free(void* p);
-
 // ---------------------------------------------------------------------------
 // Tensor maps
 // ---------------------------------------------------------------------------

@@ -887,7 +887,7 @@ extern "C" int gm_levin_store_alloc(gm_levin_store* st, int W, int H, int precis
     const size_t b32 = (12 * plane * 4 + 255) & ~(size_t)255;
     const size_t b1 = (plane * 4 + 255) & ~(size_t)255;
     unsigned char* m = nullptr;
-    if (gm_store_malloc((void**)&m, lo_bytes + b32 + 4 * b1) != cudaSuccess) {
+    if (cudaMalloc((void**)&m, lo_bytes + b32 + 4 * b1) != cudaSuccess) {
         cudaGetLastError();
         gm_set_error_msg("store allocation failed");
         return GM_ERR_NOMEM;
@@ -905,7 +905,10 @@ extern "C" int gm_levin_store_alloc(gm_levin_store* st, int W, int H, int precis
 extern "C" int gm_levin_store_free(gm_levin_store* st)
 {
     if (!st) return GM_ERR_INVALID;
-    if (st->owns && st->w32) gm_store_free(st->w32);
+    // cudaFree waits for every use of the block by itself, on any device and
+    // while other threads capture; a pool's free would need a wait of the
+    // device, which a capture anywhere on it refuses and is broken by.
+    if (st->owns && st->w32) cudaFree(st->w32);
     memset(st, 0, sizeof(*st));
     return GM_OK;
 }
