@@ -48,6 +48,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "gm_graph_cache.h"
 #include "gm_internal.cuh"
 
 namespace gm {
@@ -1564,7 +1565,7 @@ static size_t carve(const Plan& pl, int P0, char* base, Args* a)
 
 // Per-device solver slots: each has a grow-only workspace, capture streams,
 // an execution stream (for batches), pinned state for the read-back, timing
-// events and a cache of instantiated graphs.  Single solves use slot 0;
+// events and a cache of instantiated graphs (gm_graph_cache.h).  Single solves use slot 0;
 // gm_levin_solve_mg_many spreads its images over the slots.
 //
 // A graph serves any buffers of its shape and parameters: the kernels that use
@@ -1606,7 +1607,6 @@ struct Dev {
 };
 
 constexpr int kSlots = 8;        // concurrent solves of gm_levin_solve_mg_many
-constexpr int kGraphCache = 16;  // instantiated graphs kept per slot
 
 // GM_MG_GRAPH=0 selects the host-driven loop (the same kernels launched
 // one by one, the done flag read every 4 iterations), e.g. for profilers
@@ -2077,7 +2077,8 @@ static void bind_fields(Args& a, const Args* src)
 }
 
 // Gives the graph the buffers of solve a.  (Launches that are already enqueued
-// keep theirs.)
+// keep theirs.)  After a failure the graph is of no use: its nodes may have
+// two solves' buffers.
 static int rebind(Graph& g, const Args& a, const FineMaps& fm)
 {
     Args b = g.launch;
@@ -2109,51 +2110,39 @@ static int rebind(Graph& g, const Args& a, const FineMaps& fm)
     return GM_OK;
 }
 
-// The graph of solve a on slot d: one bound to it already, else one of its
-// shape, given its buffers, else a new one.  A program that goes round a few
-// sets of buffers gets a graph for each (up to kSameShape) once the bindings
-// have cost as much as a capture.  The reference is valid until the next call.
-constexpr int kSameShape = 4, kRebindsPerCapture = 50;
+// A solve, as the cache of graphs asks about it.
+template <class T>
+struct GraphOps {
+    Dev& d;
+    const Args& a;
+    const FineMaps& fm;
+    int tcode;
+    Args shape;
+
+    GraphOps(Dev& dev, const Args& args, const FineMaps& maps, int tc) : d(dev), a(args), fm(maps), tcode(tc)
+    {
+        memcpy(&shape, &a, sizeof(Args));
+        bind_fields(shape, nullptr);
+    }
+    bool same_shape(const Graph& g) const { return g.tcode == tcode && memcmp(&g.shape, &shape, sizeof(Args)) == 0; }
+    bool bound(const Graph& g) const { return memcmp(&g.key, &a, sizeof(Args)) == 0; }
+    int bind(Graph& g) const { return rebind(g, a, fm); }
+    int build(Graph& g) const
+    {
+        GM_TRY(build_graph<T>(d, a, fm, g));
+        memcpy(&g.key, &a, sizeof(Args));
+        memcpy(&g.shape, &shape, sizeof(Args));
+        g.tcode = tcode;
+        return GM_OK;
+    }
+    void drop(Graph& g) const { free_graph(g); }
+};
+
+// The graph of solve a on slot d, valid until the next call.
 template <class T>
 static int graph_for(Dev& d, const Args& a, const FineMaps& fm, int tcode, Graph** out)
 {
-    Args shape;
-    memcpy(&shape, &a, sizeof(Args));
-    bind_fields(shape, nullptr);
-    Graph* old = nullptr;
-    int same = 0, rebinds = 0;
-    for (Graph& g : d.graphs) {
-        if (g.tcode != tcode || memcmp(&g.shape, &shape, sizeof(Args)) != 0) continue;
-        if (memcmp(&g.key, &a, sizeof(Args)) == 0) {
-            g.used = ++d.clock;
-            *out = &g;
-            return GM_OK;
-        }
-        ++same;
-        rebinds += g.rebinds;
-        if (!old || g.used < old->used) old = &g;
-    }
-    if (old && (same >= kSameShape || rebinds < same * kRebindsPerCapture) && rebind(*old, a, fm) == GM_OK) {
-        old->rebinds += 1;
-        old->used = ++d.clock;
-        *out = old;
-        return GM_OK;
-    }
-    Graph g = {};
-    GM_TRY(build_graph<T>(d, a, fm, g));
-    memcpy(&g.key, &a, sizeof(Args));
-    memcpy(&g.shape, &shape, sizeof(Args));
-    g.tcode = tcode;
-    g.used = ++d.clock;
-    if (d.graphs.size() >= (size_t)kGraphCache) {
-        auto lru = std::min_element(d.graphs.begin(), d.graphs.end(),
-                                    [](const Graph& x, const Graph& y) { return x.used < y.used; });
-        free_graph(*lru);
-        d.graphs.erase(lru);
-    }
-    d.graphs.push_back(std::move(g));
-    *out = &d.graphs.back();
-    return GM_OK;
+    return cached_graph(d.graphs, d.clock, GraphOps<T>(d, a, fm, tcode), out);
 }
 
 template <class T>
