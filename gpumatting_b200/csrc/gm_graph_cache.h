@@ -1,6 +1,6 @@
-// gm_graph_cache.h -- which captured graph serves a solve: host logic only, no
-// CUDA, so that its error paths can be tested without a GPU
-// (tests/c/test_graph_cache.cpp).
+// gm_graph_cache.h -- which captured graph serves a solve, and the steps of a
+// batch of solves: host logic only, no CUDA, so that its error paths can be
+// tested without a GPU (tests/c/test_graph_cache.cpp).
 #ifndef GM_GRAPH_CACHE_H
 #define GM_GRAPH_CACHE_H
 
@@ -63,6 +63,29 @@ int cached_graph(std::vector<G>& graphs, unsigned long long& clock, Ops&& ops, G
     graphs.push_back(std::move(g));
     *out = &graphs.back();
     return 0;
+}
+
+// A batch of n solves on several streams.  Ops: ready(k), solve k has a graph;
+// begin(), the streams follow the caller's; launch(k); join(), the caller's stream
+// follows them and has been waited for (0: done).  A solve in flight writes the
+// caller's vectors and uses its slot's workspace, so after a failure it is
+// waited for (drain()) before the error is returned; *launched tells a failure
+// that came before any launch, after which another way may be tried.
+template <class Ops>
+int run_images(int n, Ops&& ops, bool* launched)
+{
+    *launched = false;
+    for (int k = 0; k < n; ++k)
+        if (const int rc = ops.ready(k)) return rc;
+    int rc = ops.begin();
+    if (rc != 0) return rc;
+    for (int k = 0; k < n && rc == 0; ++k) {
+        *launched = true;
+        rc = ops.launch(k);
+    }
+    if (rc == 0) rc = ops.join();
+    if (rc != 0) ops.drain();
+    return rc;
 }
 
 }  // namespace gm

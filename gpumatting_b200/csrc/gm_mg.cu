@@ -2203,45 +2203,71 @@ struct Item {
     int slot;
 };
 
-// Launches every image's graph on the execution stream of its slot, forked
-// from and joined back to st, and copies each
-// image's final state to pinned memory on the same stream.  The images of one
-// slot run one after another (they share its workspace); different slots run
-// concurrently.  One host synchronisation for the whole batch.
+// Every image's graph goes to the execution stream of its slot, forked
+// from and joined back to st, and each image's final state to pinned memory on
+// the same stream.  The images of one slot run one after another (they share
+// its workspace); different slots run concurrently.  One host synchronisation
+// for the whole batch.
 template <class T>
-static int run_many(Dev* slots, int K, std::vector<Item>& items, int tcode, cudaStream_t st, float* ms)
-{
-    const int n = (int)items.size();
-    Dev& d0 = slots[0];
-    for (int k = 0; k < n; ++k) {  // captures come before the timing
+struct ManyOps {
+    Dev* slots;
+    int K;
+    std::vector<Item>& items;
+    int tcode;
+    cudaStream_t st;
+    float* ms;
+
+    int graph(int k, Graph** g) const
+    {
+        return graph_for<T>(slots[items[k].slot], items[k].a, items[k].fm, tcode, g);
+    }
+    int ready(int k) const  // captures come before the timing
+    {
         Graph* g = nullptr;
-        GM_TRY(graph_for<T>(slots[items[k].slot], items[k].a, items[k].fm, tcode, &g));
+        return graph(k, &g);
     }
-    if (d0.pin_n < n) {
-        if (d0.pin) cudaFreeHost(d0.pin);
-        d0.pin = nullptr;
-        d0.pin_n = 0;
-        GM_CUDA_TRY(cudaMallocHost((void**)&d0.pin, (size_t)n * sizeof(State)));
-        d0.pin_n = n;
+    int begin() const
+    {
+        Dev& d0 = slots[0];
+        const int n = (int)items.size();
+        if (d0.pin_n < n) {
+            if (d0.pin) cudaFreeHost(d0.pin);
+            d0.pin = nullptr;
+            d0.pin_n = 0;
+            GM_CUDA_TRY(cudaMallocHost((void**)&d0.pin, (size_t)n * sizeof(State)));
+            d0.pin_n = n;
+        }
+        GM_CUDA_TRY(cudaEventRecord(d0.e0, st));
+        for (int j = 0; j < K; ++j) GM_CUDA_TRY(cudaStreamWaitEvent(slots[j].run, d0.e0, 0));
+        d0.cond_ok = 1;
+        return GM_OK;
     }
-    GM_CUDA_TRY(cudaEventRecord(d0.e0, st));
-    for (int j = 0; j < K; ++j) GM_CUDA_TRY(cudaStreamWaitEvent(slots[j].run, d0.e0, 0));
-    for (int k = 0; k < n; ++k) {
+    int launch(int k) const
+    {
         Dev& d = slots[items[k].slot];
         Graph* g = nullptr;
-        GM_TRY(graph_for<T>(d, items[k].a, items[k].fm, tcode, &g));
+        GM_TRY(graph(k, &g));
         GM_CUDA_TRY(cudaGraphLaunch(g->exec, d.run));
-        GM_CUDA_TRY(cudaMemcpyAsync(d0.pin + k, items[k].a.st, sizeof(State), cudaMemcpyDeviceToHost, d.run));
+        GM_CUDA_TRY(cudaMemcpyAsync(slots[0].pin + k, items[k].a.st, sizeof(State), cudaMemcpyDeviceToHost, d.run));
+        return GM_OK;
     }
-    for (int j = 0; j < K; ++j) {
-        GM_CUDA_TRY(cudaEventRecord(slots[j].e1, slots[j].run));
-        GM_CUDA_TRY(cudaStreamWaitEvent(st, slots[j].e1, 0));
+    int join() const
+    {
+        for (int j = 0; j < K; ++j) {
+            GM_CUDA_TRY(cudaEventRecord(slots[j].e1, slots[j].run));
+            GM_CUDA_TRY(cudaStreamWaitEvent(st, slots[j].e1, 0));
+        }
+        GM_CUDA_TRY(cudaEventRecord(slots[0].e2, st));
+        GM_CUDA_TRY(cudaStreamSynchronize(st));
+        cudaEventElapsedTime(ms, slots[0].e0, slots[0].e2);
+        return GM_OK;
     }
-    GM_CUDA_TRY(cudaEventRecord(d0.e2, st));
-    GM_CUDA_TRY(cudaStreamSynchronize(st));
-    cudaEventElapsedTime(ms, d0.e0, d0.e2);
-    return GM_OK;
-}
+    void drain() const
+    {
+        for (int j = 0; j < K; ++j) cudaStreamSynchronize(slots[j].run);
+        cudaGetLastError();
+    }
+};
 
 // Fills the level-0 fields and the carve of an Args for the store.
 static int prepare(const gm_levin_store* store, int use_low, Plan& pl, Args& a, size_t* bytes, int* tcode)
@@ -2460,10 +2486,11 @@ extern "C" int gm_levin_solve_mg_many(const gm_levin_store* const* stores, float
     } else {
         float ms = 0.f;
         int rc;
-        if (tcode == 1) rc = run_many<__half>(slots, K, items, tcode, st, &ms);
-        else if (tcode == 2) rc = run_many<__nv_bfloat16>(slots, K, items, tcode, st, &ms);
-        else rc = run_many<float>(slots, K, items, tcode, st, &ms);
-        if (rc != GM_OK && slots[0].cond_ok == -1) {
+        bool launched = false;
+        if (tcode == 1) rc = run_images(count, ManyOps<__half>{slots, K, items, tcode, st, &ms}, &launched);
+        else if (tcode == 2) rc = run_images(count, ManyOps<__nv_bfloat16>{slots, K, items, tcode, st, &ms}, &launched);
+        else rc = run_images(count, ManyOps<float>{slots, K, items, tcode, st, &ms}, &launched);
+        if (rc != GM_OK && !launched && slots[0].cond_ok == -1) {
             // the first capture failed: no conditional graphs here, so solve
             // the images one after another with the host-driven loop
             slots[0].cond_ok = 0;
@@ -2485,7 +2512,6 @@ extern "C" int gm_levin_solve_mg_many(const gm_levin_store* const* stores, float
             return worst;
         }
         if (rc != GM_OK) return rc;
-        slots[0].cond_ok = 1;
         for (int k = 0; k < count; ++k) {
             if (infos) fill_info(&infos[k], slots[0].pin[k], ms, items[k].pl.L + 1);
             worst = std::max(worst, slots[0].pin[k].status);

@@ -1,6 +1,6 @@
 // The cache of captured solves (csrc/gm_graph_cache.h) with a fake capture: a
 // graph has ten nodes, each with the buffer it was given last, and setting a
-// node can be made to fail.
+// node can be made to fail.  And the steps of a batch with one that fails.
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -100,10 +100,48 @@ static void many_shapes()
     CHECK((int)c.graphs.size() == (int)gm::kGraphCache);
 }
 
+// A batch whose step number `fail_at` fails: nothing is left in flight, and a
+// failure counts as one before the launches only where nothing was launched.
+struct Batch {
+    int n, fail_at;
+    int step = 0, launches = 0, in_flight = 0;
+    int next() { return step++ == fail_at ? 7 : 0; }
+    int ready(int) { return next(); }
+    int begin() { return next(); }
+    int launch(int)
+    {
+        ++launches;
+        ++in_flight;  // also where the call that follows the launch fails
+        return next();
+    }
+    int join()
+    {
+        const int rc = next();
+        if (rc == 0) in_flight = 0;
+        return rc;
+    }
+    void drain() { in_flight = 0; }
+};
+
+static void failing_batch()
+{
+    for (int n = 1; n < 5; ++n)
+        for (int at = -1; at < 2 * n + 2; ++at) {
+            Batch b{n, at};
+            bool launched = false;
+            const int rc = gm::run_images(n, b, &launched);
+            CHECK(rc == (at < 0 ? 0 : 7));
+            CHECK(b.in_flight == 0);
+            CHECK(launched == (b.launches > 0));
+            CHECK(at < 0 ? b.launches == n : b.launches <= n);
+        }
+}
+
 int main()
 {
     failing_bind();
     many_shapes();
+    failing_batch();
     std::printf("Test PASSED\n");
     return 0;
 }
