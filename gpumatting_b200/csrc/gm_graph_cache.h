@@ -12,18 +12,21 @@
 namespace gm {
 
 constexpr size_t kGraphCache = 16;  // instantiated graphs kept
+// Graphs of one shape that single solves go round, and bindings (10-25 us) that
+// cost as much as a capture (1-2 ms).  A batch goes round as many as it has
+// images of the shape on a slot.
 constexpr int kSameShape = 4, kRebindsPerCapture = 50;
 
 // The graph of a solve: one bound to its buffers already, else one of its
 // shape, given its buffers, else a new one.  A program that goes round a few
-// sets of buffers gets a graph for each (up to kSameShape) once the bindings
+// sets of buffers gets a graph for each (up to `keep` of them) once the bindings
 // have cost as much as a capture.
 //
 // G has `used` and `rebinds`.  Ops answers for the solve: same_shape(g), bound(g),
 // bind(g) and build(g) (0: done) and drop(g), which frees g's graph.  The result
 // is valid until the next call.
 template <class G, class Ops>
-int cached_graph(std::vector<G>& graphs, unsigned long long& clock, Ops&& ops, G** out)
+int cached_graph(std::vector<G>& graphs, unsigned long long& clock, int keep, Ops&& ops, G** out)
 {
     size_t old = graphs.size();
     int same = 0, rebinds = 0;
@@ -39,7 +42,7 @@ int cached_graph(std::vector<G>& graphs, unsigned long long& clock, Ops&& ops, G
         rebinds += g.rebinds;
         if (old == graphs.size() || g.used < graphs[old].used) old = i;
     }
-    if (same > 0 && (same >= kSameShape || rebinds < same * kRebindsPerCapture)) {
+    if (same > 0 && (same >= keep || rebinds < same * kRebindsPerCapture)) {
         G& g = graphs[old];
         if (ops.bind(g) == 0) {
             g.rebinds += 1;
@@ -63,6 +66,18 @@ int cached_graph(std::vector<G>& graphs, unsigned long long& clock, Ops&& ops, G
     graphs.push_back(std::move(g));
     *out = &graphs.back();
     return 0;
+}
+
+// A graph of the solve's shape, whatever it is bound to; in a full cache none is
+// captured yet, where it could push out one that is about to be launched.
+template <class G, class Ops>
+int ready_graph(std::vector<G>& graphs, unsigned long long& clock, int keep, Ops&& ops)
+{
+    if (graphs.size() >= kGraphCache) return 0;
+    for (const G& g : graphs)
+        if (ops.same_shape(g)) return 0;
+    G* g = nullptr;
+    return cached_graph(graphs, clock, keep, ops, &g);
 }
 
 // A batch of n solves on several streams.  Ops: ready(k), solve k has a graph;

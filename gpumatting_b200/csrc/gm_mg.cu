@@ -40,10 +40,12 @@
 // chained with programmatic dependent launch.  gm_levin_solve_mg_many runs
 // many such solves on concurrent streams.
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -2138,20 +2140,13 @@ struct GraphOps {
     void drop(Graph& g) const { free_graph(g); }
 };
 
-// The graph of solve a on slot d, valid until the next call.
-template <class T>
-static int graph_for(Dev& d, const Args& a, const FineMaps& fm, int tcode, Graph** out)
-{
-    return cached_graph(d.graphs, d.clock, GraphOps<T>(d, a, fm, tcode), out);
-}
-
 template <class T>
 static int run(Dev& d, const Args& a0, const FineMaps& fm, int tcode, cudaStream_t st, float* ms)
 {
     Args a = a0;
     if (d.cond_ok != 0 && graph_enabled()) {
         Graph* hit = nullptr;
-        const int rc = graph_for<T>(d, a, fm, tcode, &hit);
+        const int rc = cached_graph(d.graphs, d.clock, kSameShape, GraphOps<T>(d, a, fm, tcode), &hit);
         if (rc == GM_OK) {
             d.cond_ok = 1;
         } else if (d.cond_ok == -1) {
@@ -2201,6 +2196,7 @@ struct Item {
     size_t bytes;
     FineMaps fm;
     int slot;
+    int same;  // images of this size on the slot
 };
 
 // Every image's graph goes to the execution stream of its slot, forked
@@ -2217,14 +2213,11 @@ struct ManyOps {
     cudaStream_t st;
     float* ms;
 
-    int graph(int k, Graph** g) const
+    int keep(int k) const { return std::max(kSameShape, std::min(items[k].same, (int)kGraphCache)); }
+    int ready(int k) const
     {
-        return graph_for<T>(slots[items[k].slot], items[k].a, items[k].fm, tcode, g);
-    }
-    int ready(int k) const  // captures come before the timing
-    {
-        Graph* g = nullptr;
-        return graph(k, &g);
+        Dev& d = slots[items[k].slot];
+        return ready_graph(d.graphs, d.clock, keep(k), GraphOps<T>(d, items[k].a, items[k].fm, tcode));
     }
     int begin() const
     {
@@ -2246,7 +2239,7 @@ struct ManyOps {
     {
         Dev& d = slots[items[k].slot];
         Graph* g = nullptr;
-        GM_TRY(graph(k, &g));
+        GM_TRY(cached_graph(d.graphs, d.clock, keep(k), GraphOps<T>(d, items[k].a, items[k].fm, tcode), &g));
         GM_CUDA_TRY(cudaGraphLaunch(g->exec, d.run));
         GM_CUDA_TRY(cudaMemcpyAsync(slots[0].pin + k, items[k].a.st, sizeof(State), cudaMemcpyDeviceToHost, d.run));
         return GM_OK;
@@ -2444,6 +2437,9 @@ extern "C" int gm_levin_solve_mg_many(const gm_levin_store* const* stores, float
             items[k].slot = j;
             load[j] += cost(k);
         }
+        std::map<std::array<int, 3>, int> same;
+        for (const Item& x : items) ++same[{x.slot, x.a.W, x.a.H}];
+        for (Item& x : items) x.same = same[{x.slot, x.a.W, x.a.H}];
     }
     for (int j = 0; j < K; ++j) {
         size_t need = 0;

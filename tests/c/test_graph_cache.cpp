@@ -1,6 +1,7 @@
 // The cache of captured solves (csrc/gm_graph_cache.h) with a fake capture: a
 // graph has ten nodes, each with the buffer it was given last, and setting a
 // node can be made to fail.  And the steps of a batch with one that fails.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -59,7 +60,7 @@ struct Cache {
     bool launch(int shape, int buffer, bool build_fails = false)
     {
         Graph* g = nullptr;
-        if (gm::cached_graph(graphs, clock, Solve{shape, buffer, build_fails}, &g) != 0) return false;
+        if (gm::cached_graph(graphs, clock, gm::kSameShape, Solve{shape, buffer, build_fails}, &g) != 0) return false;
         CHECK(g != nullptr && g->shape == shape);
         for (int n : g->node) CHECK(n == buffer);
         CHECK((int)graphs.size() == g_alive && graphs.size() <= gm::kGraphCache);
@@ -98,6 +99,41 @@ static void many_shapes()
     Cache c;
     for (int i = 0; i < 2000; ++i) CHECK(c.launch(i % 23, i % 7));
     CHECK((int)c.graphs.size() == (int)gm::kGraphCache);
+}
+
+// A repeated batch with n images of one shape on a slot: at most one binding an
+// image and call, and none once each has a graph of its own, where the cache
+// holds that many.
+static void repeated_batch()
+{
+    for (int n = 1; n <= 20; ++n) {
+        Cache c;
+        const int keep = std::min(n, (int)gm::kGraphCache), builds = g_builds;
+        int sets = 0;
+        for (int call = 0; call < 1000; ++call) {
+            const int before = g_sets;
+            for (int k = 0; k < n; ++k) CHECK(gm::ready_graph(c.graphs, c.clock, keep, Solve{1, k}) == 0);
+            CHECK(g_sets == before);
+            for (int k = 0; k < n; ++k) {
+                Graph* g = nullptr;
+                CHECK(gm::cached_graph(c.graphs, c.clock, keep, Solve{1, k}, &g) == 0 && g->key == k);
+            }
+            sets = g_sets - before;
+            CHECK(sets <= n * kNodes);
+        }
+        CHECK(n > keep || sets == 0);
+        CHECK(g_builds - builds <= (int)gm::kGraphCache);
+    }
+    // images of n shapes each: at most one capture an image and call
+    for (int n = 1; n <= 40; ++n) {
+        Cache c;
+        for (int call = 0; call < 5; ++call) {
+            const int before = g_builds;
+            for (int k = 0; k < n; ++k) CHECK(gm::ready_graph(c.graphs, c.clock, 1, Solve{k, k}) == 0);
+            for (int k = 0; k < n; ++k) CHECK(c.launch(k, k));
+            CHECK(g_builds - before <= (call > 0 && n <= (int)gm::kGraphCache ? 0 : n));
+        }
+    }
 }
 
 // A batch whose step number `fail_at` fails: nothing is left in flight, and a
@@ -141,6 +177,7 @@ int main()
 {
     failing_bind();
     many_shapes();
+    repeated_batch();
     failing_batch();
     std::printf("Test PASSED\n");
     return 0;

@@ -422,6 +422,27 @@ def test_mg_graph_serves_other_buffers(orc):
         assert torch.equal(solve(i % 4, bufs[i % 5]), first[i % 4]), i
 
 
+def test_mg_batch_of_equal_images():
+    """More images of one size than a slot keeps graphs of a shape for single
+    solves, on new vectors in every call: each image's own matte, bit for bit."""
+    torch = torch_cuda()
+    from gpumatting_b200 import api
+
+    W, H, n = 40, 31, 41  # six on one of the eight slots
+    bt = api.LevinBatch([(W, H)] * n, "fp16")
+    want = []
+    for k in range(n):
+        img, scr = (torch.from_numpy(x).cuda() for x in edge_image(W, H, k))
+        bt.assemble(k, img, scr, eps=1e-5)
+        want.append(torch.full((H, W), 0.5, device="cuda"))
+        api.LevinStore(W, H, "fp16").assemble(img, scr, eps=1e-5).solve(want[k], "mg", rtol=0.0, max_iters=5)
+    assert not torch.equal(want[0], want[1])
+    for call in range(80):
+        alphas = [torch.full((H, W), 0.5, device="cuda") for _ in range(n)]
+        bt.solve(alphas, "mg", rtol=0.0, max_iters=5)
+        assert all(torch.equal(a, w) for a, w in zip(alphas, want)), call
+
+
 def test_batch_solve_with_mg(orc):
     """gm_batch_solve with GM_SOLVER_MG gives every image of the canvas its own
     one-graph MG solve (concurrent streams): each result matches, bit for bit
