@@ -162,7 +162,11 @@ template <class T> __device__ __forceinline__ float tof(T v) { return Cvt<T>::to
 // programmatic stream serialisation, waits for its predecessor's completion
 // (and memory), and lets its successor start launching only then.  So when a
 // kernel starts, all kernels before its predecessor are complete: ahead of the
-// wait it may read what those wrote, and only that.  This hides the launch gap
+// wait it may read what those wrote, and only that.  Their writes are in L2 by
+// then (the predecessor's wait is for that too); what changes from iteration to
+// iteration is read from there (__ldcg, TMA), because no wait of the reading
+// kernel's own has dropped older lines from L1 yet.  What the set-up wrote is
+// constant in the iterations, and plain loads do.  This hides the launch gap
 // between the many short kernels of a V-cycle.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -287,9 +291,11 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
     // predecessor started after them) is read ahead of the wait for it.
     State* st = a.st;
     const int W = a.W, H = a.H, P = a.P;
-    const int it = st->iter;
-    const bool fold = st->fold_at == it;  // a replacement ran: move the increment into x
-    const float* pn = (it & 1) ? a.p0 : a.p1;
+    __shared__ int s_it, s_fold;
+    if (threadIdx.x == 0) {  // (one thread: every warp's request for the one line would queue up in L2)
+        s_it = __ldcg(&st->iter);
+        s_fold = __ldcg(&st->fold_at);
+    }
     const int qpr = (W + 3) / 4;
     const size_t nq = (size_t)qpr * H, step = (size_t)gridDim.x * kThreads;
     struct Quad {
@@ -300,9 +306,10 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
     auto load_old = [&](Quad& d, size_t qi) {
         d.x = (int)(qi % qpr) * 4;
         d.o = (qi / qpr) * P + d.x;
-        d.r = *reinterpret_cast<const float4*>(a.r + d.o);
-        d.xi = *reinterpret_cast<const float4*>(a.xinc + d.o);
+        d.r = __ldcg(reinterpret_cast<const float4*>(a.r + d.o));
+        d.xi = __ldcg(reinterpret_cast<const float4*>(a.xinc + d.o));
     };
+    const float* pn = nullptr;
     auto load_new = [&](Quad& d) {
         d.p = *reinterpret_cast<const float4*>(pn + d.o);
         d.q = *reinterpret_cast<const float4*>(a.q + d.o);
@@ -310,6 +317,10 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
     size_t qi = (size_t)blockIdx.x * kThreads + threadIdx.x;
     Quad c, n;
     if (qi < nq) load_old(c, qi);
+    __syncthreads();
+    const int it = s_it;
+    const bool fold = s_fold == it;  // a replacement ran: move the increment into x
+    pn = (it & 1) ? a.p0 : a.p1;
     pdl_enter();
     if (qi < nq) load_new(c);
     const double rz = st->rz[it & 1];
@@ -785,6 +796,10 @@ __global__ void __launch_bounds__(32 * ROWS, 1)
     const int W = F.W, H = F.H, P = F.P, tid = threadIdx.x, G = gridDim.x;
     const int ntx = (W + kFTW - 1) / kFTW, ntiles = ntx * ((H + TH - 1) / TH);
     const int t0 = blockIdx.x;
+    State* st = a.st;
+    // (of FM_SPMV's predecessors only those long complete write iter; one thread
+    // reads it, as every warp's request for the one line would queue up in L2)
+    int it = MODE == FM_SPMV && tid == 0 ? __ldcg(&st->iter) : 0;
     if (tid == 0) {
         mbar_init(&full[0], 1);
         mbar_init(&full[1], 1);
@@ -808,14 +823,9 @@ __global__ void __launch_bounds__(32 * ROWS, 1)
             mbar_expect_tx(&full[k], (uint32_t)LY::PB);
             issue_planes(t0 + k * G, k);
         }
-    State* st = a.st;
-    // (of FM_SPMV's predecessors only those long complete write iter)
-    const int it = MODE == FM_SPMV ? st->iter : 0;
-    const bool first = it == 0;
     pdl_enter();
     const float om = a.omega, sc = a.scale;
-    const CUtensorMap* mv1 = MODE == FM_SPMV ? ((it & 1) ? &tm.m[3] : &tm.m[2]) : &tm.m[2];
-    float* pnew = (it & 1) ? a.p0 : a.p1;
+    const CUtensorMap* mv1 = MODE == FM_SPMV && (it & 1) ? &tm.m[3] : &tm.m[2];  // (for thread 0)
     const Lev& C = a.lev[l + 1];
     auto issue_vectors = [&](int t, int s) {
         const int u0 = (t % ntx) * kFTW, v0 = (t / ntx) * TH;
@@ -844,7 +854,8 @@ __global__ void __launch_bounds__(32 * ROWS, 1)
     float beta = 0.f;
     const bool summing = MODE == FM_SPMV || (MODE == FM_DOWN && pending);
     __shared__ double s_sum;
-    __shared__ int s_stop;
+    __shared__ int s_stop, s_it;
+    if (tid == 0) s_it = it;
     if (summing && tid >= 32 && tid < 64) {
         const double t = MODE == FM_SPMV ? warp_sum_range(a.parts + (size_t)S_RZ * kMaxParts, 0, a.n_rz)
                                          : warp_sum_range(a.parts + (size_t)S_RR * kMaxParts, 0, a.n_rr);
@@ -858,6 +869,9 @@ __global__ void __launch_bounds__(32 * ROWS, 1)
         drain();
         return;
     }
+    it = s_it;
+    const bool first = it == 0;
+    float* pnew = (it & 1) ? a.p0 : a.p1;
     if (summing) {
         const double sum = s_sum;
         const bool lead = blockIdx.x == 0 && tid == 0;
@@ -1173,6 +1187,17 @@ __global__ void __launch_bounds__(kPairThreads) mg_pair_up_kernel(Args a, int l)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int mx0 = (t % tx) * kPW1, my0 = (t / tx) * kPH1;
         const int fx0 = 2 * mx0, fy0 = 2 * my0;
+        float gb[NY], fb[NF];
+#pragma unroll
+        for (int j = 0; j < NY; ++j) {
+            const int i = tid + j * kPairThreads, x = mx0 - 2 + i % YW, y = my0 - 2 + i / YW;
+            gb[j] = i < YW * YH && x >= 0 && x < G.W && y >= 0 && y < G.H ? __ldcg(G.b + (size_t)y * G.P + x) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < NF; ++j) {
+            const int i = tid + j * kPairThreads, x = fx0 - 1 + i % FW, y = fy0 - 1 + i / FW;
+            fb[j] = i < FW * FH && x >= 0 && x < F.W && y >= 0 && y < F.H ? __ldcg(F.b + (size_t)y * F.P + x) : 0.f;
+        }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             stage<YW, YH - 1>(cm + k * (YH - 1) * YW, static_cast<const float*>(G.c) + k * G.ps, G.P, G.W, G.H, mx0 - 2,
@@ -1180,9 +1205,7 @@ __global__ void __launch_bounds__(kPairThreads) mg_pair_up_kernel(Args a, int l)
             stage<FW, FH - 1>(cf + k * (FH - 1) * FW, static_cast<const float*>(F.c) + k * F.ps, F.P, F.W, F.H, fx0 - 1,
                               fy0 - 1);
         }
-        stage<YW, YH>(bm, G.b, G.P, G.W, G.H, mx0 - 2, my0 - 2);
         stage<YW, YH>(dm, G.Di, G.P, G.W, G.H, mx0 - 2, my0 - 2);
-        stage<FW, FH>(bf, F.b, F.P, F.W, F.H, fx0 - 1, fy0 - 1);
         stage<FW, FH>(df, F.Di, F.P, F.W, F.H, fx0 - 1, fy0 - 1);
         if (!waited) {
             pdl_enter();
@@ -1200,8 +1223,14 @@ __global__ void __launch_bounds__(kPairThreads) mg_pair_up_kernel(Args a, int l)
 #pragma unroll
         for (int j = 0; j < NY; ++j) {  // (each thread reads what it staged itself)
             const int i = tid + j * kPairThreads;
-            if (i < YW * YH) ym[i] = dm[i] > 0.f ? fmaf(sc, xc[j], om * bm[i] * dm[i]) : 0.f;
+            if (i < YW * YH) {
+                ym[i] = dm[i] > 0.f ? fmaf(sc, xc[j], om * gb[j] * dm[i]) : 0.f;
+                bm[i] = gb[j];
+            }
         }
+#pragma unroll
+        for (int j = 0; j < NF; ++j)
+            if (tid + j * kPairThreads < FW * FH) bf[tid + j * kPairThreads] = fb[j];
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < NM; ++j) {
