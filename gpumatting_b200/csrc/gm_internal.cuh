@@ -134,13 +134,17 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 }
 
 // L2 policy of the plane loads.  The planes of an operator are read once or
-// twice per iteration, the vectors by every kernel: where the vectors fit L2
-// but vectors and planes together do not, the planes' lines are marked to
-// leave first.  Us per iteration without and with: fused CG, FP32 store, 1080p
-// 35.8 / 31.7, FP16 28.5 / 28.3, within 0.5 % up to 1400 x 760; multigrid with the
-// FP32 outer product 1501 x 703 61 / 58, 1080p 93.0 / 91.0.  Where the vectors do not fit either, the marked
-// lines only lose what reuse there was (4096^2: multigrid 474 / 491, a CG
-// replacement 2x slower), and smaller problems fit whole.
+// twice per iteration, the vectors by every kernel: up to the size whose vectors
+// fit L2, the planes' lines are marked to leave first.  Us per iteration
+// without and with, fused CG: FP32 store 1080p 37.8 / 33.5, 1501 x 1000 29.2 / 27.8,
+// 1280 x 1024 25.9 / 25.7, FP16 1080p 30.2 / 29.8; multigrid with FP32 planes
+// 1080p 121.8 / 118.7, 1501 x 1000 102.9 / 99.5, 130 x 1900 52.8 / 49.6, FP16 94.5 / 93.8
+// at 1080p.  Where vectors and planes fit together it mostly changes nothing (ten
+// sizes from 130 x 97: at worst 0.1 % slower with it), so the rule has no lower
+// limit; nor does it count the solves of a batch, of which eight at once take the
+// same time either way (within 2 %; 8 x 1000 x 750, FP32: 17.9 / 17.5 ms).  Where the
+// vectors do not fit, the marked lines only lose what reuse there was (4096^2:
+// multigrid 474 / 491, a CG replacement 2x slower).
 constexpr long long kPlanesFirstMaxPixels = 3500000;  // 32 B of vectors per pixel against 126 MB of L2
 inline int planes_leave_first(long long pixels) { return pixels <= kPlanesFirstMaxPixels ? 1 : 0; }
 __device__ __forceinline__ uint64_t plane_policy(int leave_first)

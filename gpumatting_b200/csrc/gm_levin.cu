@@ -136,19 +136,22 @@ struct SymOut {
 // rows of a run repeat the couplings of the two rows above it; runs are as
 // long as one wave of CTAs allows.
 //
-// Measured with the FP16 store: 1080p RGB8 450 -> 117 us, 4096^2 850 us (83 B
-// written per pixel are 26 and 215 us); FP32 store, 4001 x 2999: 2,400 -> 500
-// (RGB8), 560 us (float).  Bound by instruction issue at 12 warps per SM (about 60
-// % of the slots, FP64 pipe 37 %).  Forms before: windows in shared memory 156 us
+// Measured with the FP16 store: 1080p RGB8 450 -> 117 us, 4096^2 4.3 -> 0.85 ms in a
+// row, 0.96-1.08 where another kernel's data has to leave L2 first (88 B written
+// per pixel are 28 and 225 us); FP32 store, 4001 x 2999: 2,400 -> 500 (RGB8), 560
+// us (float).  Bound by instruction issue at 12 warps per SM (about 60 % of the
+// slots, FP64 pipe 37 %).  Forms before: windows in shared memory 156 us
 // (12 shared wavefronts per 32 pixels and window); all rounded couplings through a
 // shared ring for the diagonal 122.
 constexpr int kAT = 128;              // threads = window columns
 constexpr int kAW = kAT - 2;          // output columns per CTA
 constexpr int kAP = kAT + 4;          // row length in shared memory (two pad columns each side)
 // CTAs per SM the registers are cut for.  A float image's 27 colours and 18 row
-// sums in 64 bits spill at 168 registers (1080p: 160 us with 3 CTAs per SM, 135
-// with 2); an RGB8 image's do not (122 us with 3, 135 with 2; before the diagonal
-// moved to registers).
+// sums in 64 bits do not fit 168 registers (1080p: 160 us with 3 CTAs per SM, 135
+// with 2).  An RGB8 image's nearly do: 116 bytes a thread are spilled with a 2-byte
+// store (164 with the 25 bands), 8 with an FP32 one.  The 12 warps are worth
+// that: 122 us with 3 CTAs per SM and 135 with 2 before the diagonal's sums moved
+// to registers (4 bytes spilled then), 117 since.
 __host__ __device__ constexpr int asm_ctas(bool f32) { return f32 ? 2 : 3; }
 constexpr int kMinRows = 2;
 

@@ -386,9 +386,10 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(Args a)
 
 // True residual r = b - A x with the FP32 planes in FP64 arithmetic (runs
 // only when a replacement is due).  Four CTAs per SM hide one tile's loads
-// behind the others' arithmetic: 62 us at 1080p, 452 at 4096^2 (with 3 CTAs, or
-// with gamma and b loaded where they are used, 73 and 560; 92 B per pixel take
-// 29 and 235).  Also forms ||b||^2 on the first call.
+// behind the others' arithmetic, at the price of 32 spilled bytes a thread: 62 us
+// at 1080p, 452 at 4096^2 (with 3 CTAs, or with gamma and b loaded where they
+// are used, 73 and 560; 92 B per pixel take 29 and 235).  Also forms ||b||^2 on
+// the first call.
 __global__ void __launch_bounds__(kThreads, 4) mg_replace_kernel(Args a)
 {
     pdl_enter();
@@ -556,6 +557,8 @@ __device__ __forceinline__ TRow t_row(const Lev& F, const Lev& C, int i, double 
 // 42.1 / 37.6 / 39.2 at 317 x 211 (420 or 1080 cells), 50.7 / 47.2 / 52.6 at
 // 640 x 480 (300 or 1200), 103.8 / 106.5 / 111.1 at 1080p (510, 510, 2040): one
 // level less costs a row of 2 K doubles per warp, more than its two launches.
+// One limit for all sizes, taken for the small ones, where it gains most; the
+// figures are from before the levels above ran in pairs.
 constexpr int kDenseMax = 1300;
 
 // M_l from M_{l+1}.  A CTA forms the rows of 8 cells next to each other: their T
