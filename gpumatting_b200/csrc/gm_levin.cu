@@ -136,9 +136,9 @@ struct SymOut {
 // rows of a run repeat the couplings of the two rows above it; runs are as
 // long as one wave of CTAs allows.
 //
-// Measured with the FP16 store: 1080p RGB8 450 -> 117 us, 4096^2 4.3 -> 0.85 ms in a
-// row, 0.96-1.08 where another kernel's data has to leave L2 first (88 B written
-// per pixel are 28 and 225 us); FP32 store, 4001 x 2999: 2,400 -> 500 (RGB8), 560
+// Measured with the FP16 store: 1080p RGB8 450 -> 114 us, 4096^2 4.3 -> 0.82 ms in a
+// row, 0.95-1.05 where another kernel's data has to leave L2 first (88 B written
+// per pixel are 28 and 225 us); FP32 store, 4001 x 2999: 2,400 -> 494 (RGB8), 556
 // us (float).  Bound by instruction issue at 12 warps per SM (about 60 % of the
 // slots, FP64 pipe 37 %).  Forms before: windows in shared memory 156 us
 // (12 shared wavefronts per 32 pixels and window); all rounded couplings through a
@@ -151,7 +151,7 @@ constexpr int kAP = kAT + 4;          // row length in shared memory (two pad co
 // with 2).  An RGB8 image's nearly do: 116 bytes a thread are spilled with a 2-byte
 // store (164 with the 25 bands), 8 with an FP32 one.  The 12 warps are worth
 // that: 122 us with 3 CTAs per SM and 135 with 2 before the diagonal's sums moved
-// to registers (4 bytes spilled then), 117 since.
+// to registers (4 bytes spilled then), 114 since.
 __host__ __device__ constexpr int asm_ctas(bool f32) { return f32 ? 2 : 3; }
 constexpr int kMinRows = 2;
 
@@ -195,9 +195,13 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
         }
 
     // Colours (u - 1, u, u + 1) of row v, zero outside the image (and in an
-    // image without any window, whatever its colours hold).
+    // image without any window, whatever its colours hold): loaded for columns
+    // that are a window's centre, without a test for each (1080p FP16, RGB8 117 ->
+    // 114 us, float 134 -> 132).  A float image's for an FP32 store keep the tests:
+    // without them the kernel took 715 us instead of 556 at 4001 x 2999.
+    constexpr bool kByPixel = F32IMG && !kLow;
     const bool in[3] = {u >= 1 && u <= W, u >= 0 && u < W, u >= -1 && u < W - 1};
-    const bool any = W >= 3 && H >= 3;
+    const bool any = (kByPixel ? W >= 3 : ok_col) && H >= 3;
     auto fetch = [&](int v, Pix (&p)[9]) {
 #pragma unroll
         for (int q = 0; q < 9; ++q) p[q] = 0;
@@ -205,7 +209,7 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
             const unsigned char* row = im.data + (size_t)v * im.pitch;
 #pragma unroll
             for (int b = 0; b < 3; ++b)
-                if (in[b]) {
+                if (!kByPixel || in[b]) {
                     if constexpr (F32IMG) {
                         const float4 q = reinterpret_cast<const float4*>(row)[u - 1 + b];
                         p[3 * b] = q.x; p[3 * b + 1] = q.y; p[3 * b + 2] = q.z;
@@ -373,7 +377,11 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
         // x: column of the upper pixel less u; the lower one is du further, dv below
         auto finish = [&](int k, int x, double w9) {
             const int dv = (k + 2) / 5, du = k - 5 * dv;
-            const double w = w9 * (1.0 / 9.0);
+            // (a float image's infinities and NaN are not made zero by the zero
+            // factors of the windows outside it: couplings that leave it are cut)
+            const bool inside = !F32IMG || ((!kByPixel || x + du >= 0 || u >= 1) &&
+                                            (!kByPixel || x + du <= 0 || u + 1 < W) && (dv == 0 || r + dv < H));
+            const double w = inside ? w9 * (1.0 / 9.0) : 0.0;
             const float wf = __double2float_rn(w);
             const int row = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2 : r3));
             if (BANDS) hi[row][c + x] = wf;

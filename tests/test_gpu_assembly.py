@@ -167,3 +167,33 @@ def test_fp64_assembly_at_strip_and_run_edges(orc, W, H, prec, fmt):
     a2, b2 = api.levin_bands25(img, torch.from_numpy(scr).cuda(), eps=1e-5, gamma_value=100.0, arithmetic="fp64")
     assert np.array_equal(a2.cpu().numpy().view(np.uint32), Lm.a.cpu().numpy().view(np.uint32))
     assert np.array_equal(b2.cpu().numpy().reshape(H, W), np.where(scr == 255, 100.0, 0.0).astype(np.float32))
+
+
+@pytest.mark.parametrize("W,H,prec", [(140, 37, "fp16"), (140, 37, "fp32"), (126, 5, "bf16"), (9, 3, "fp32")])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_nonfinite_colours_stay_in_their_windows(orc, W, H, prec, bad):
+    """A non-finite colour of a float image reaches the couplings of the 3x3
+    windows that hold it and nothing else: couplings out of the image are zero
+    whatever its border holds.  The couplings of the others are the bits of the
+    image without it."""
+    torch = torch_cuda()
+    from gpumatting_b200 import api
+
+    rng = np.random.default_rng(W)
+    base = np.ones((H, W, 4), np.float32)
+    base[..., :3] = rng.random((H, W, 3))
+
+    def planes(image):
+        st = api.LevinStore(W, H, prec).assemble(torch.from_numpy(image).cuda(), eps=1e-5)
+        return [st.planes(n)[..., :W].float().cpu().numpy() for n in ("w32", "w", "d32", "d")]
+
+    clean = planes(base)
+    for x, y in [(0, 0), (W - 1, 0), (0, H - 1), (W - 1, H - 1), (1, H // 2), (W - 2, 1), (W // 2, H - 2), (W - 1, H // 2)]:
+        image = base.copy()
+        image[y, x, 1] = bad
+        fin = np.isfinite(orc.levin_sym64(np.ascontiguousarray(image[..., :3].astype(np.float64)), 1e-5).reshape(12, H, W))
+        rows = _row_diag((~fin).astype(np.float64), np.zeros(W * H), W, H).reshape(H, W) == 0.0
+        for name, got, ref in zip(("w32", "w", "d32", "d"), planes(image), clean):
+            ok = np.isfinite(got)
+            assert np.array_equal(ok, fin if name[0] == "w" else rows), (name, x, y)
+            assert np.array_equal(got[ok], ref[ok]), (name, x, y)
