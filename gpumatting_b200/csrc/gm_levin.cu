@@ -18,6 +18,8 @@
 //                      bit-identical to hostLevinLaplacian (Matting.cu:39-219).
 #include <string.h>
 
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "gm_internal.cuh"
@@ -170,9 +172,28 @@ __device__ __forceinline__ double biased_to_double(unsigned n)
     return __hiloint2double(0x43300000, (int)n) - 4503601774854144.0;  // 2^52 + 2^31
 }
 
+// What is added to the diagonal of N: e9 + rel sum(x x), with
+// e9 = 9 eps.  A window of fewer than three independent colours has a singular
+// N, and with eps = 0 (or too little to show beside N's entries in 64 bits) a
+// pivot of zero, whose reciprocal makes the window NaN.  As much is added then as
+// keeps every pivot positive in rounding, which gives the limit of small eps:
+// colours of a window lie in the range of its N, and a flat window couples its
+// pixels with 1/9.  RGB8: N is whole, at most 81 127.5^2 < 2^21, and the last pivot
+// is at least e9 N_00 with an error of 2^-51 N_00 N_22: e9 = 2^-26 is 16 times that.
+// Float: the sums err by up to 2^-49 of 9 sum(x x), 2^-47 is 4 times that; so
+// little it changes nothing where eps counts, and it is left out from 1e-10 on.
+struct Ridge {
+    double e9, rel;
+};
+static Ridge ridge_for(double eps, bool f32img)
+{
+    if (!f32img) return {std::max(9.0 * eps * (255.0 * 255.0), std::ldexp(1.0, -26)), 0.0};
+    return {std::max(9.0 * eps, 1e-60), eps < 1e-10 ? std::ldexp(9.0, -47) : 0.0};
+}
+
 template <class T, bool F32IMG, bool BANDS>
-__global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgView im, ScribView sc, double e9, int W, int H,
-                                                                       int rows, SymOut o)
+__global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgView im, ScribView sc, Ridge ridge, int W,
+                                                                       int H, int rows, SymOut o)
 {
     constexpr bool kLow = sizeof(T) == 2;
     // Two sets of nine FP64 sums do not fit beside a float image's registers
@@ -292,6 +313,8 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
             N[2] = biased_to_double(9 * s[5] - s[0] * s[2] + B); N[3] = biased_to_double(9 * s[6] - s[1] * s[1] + B);
             N[4] = biased_to_double(9 * s[7] - s[1] * s[2] + B); N[5] = biased_to_double(9 * s[8] - s[2] * s[2] + B);
         }
+        double e9 = ridge.e9;
+        if (F32IMG && ridge.rel > 0.0) e9 = fma(ridge.rel, (double)(s[3] + s[6] + s[8]), e9);
         const double s00 = N[0] + e9, s11 = N[3] + e9, s22 = N[5] + e9;
         const double c22 = fma(s00, s11, -N[1] * N[1]), c12 = fma(s00, N[4], -N[2] * N[1]),
                      c11 = fma(s00, s22, -N[2] * N[2]);
@@ -629,8 +652,7 @@ static int launch_sym3(const ImgView& im, const ScribView& sc, double eps, int W
     const int runs = max(1, asm_ctas(F32IMG) * sms / strips);
     const int rows = max(kMinRows, (H + runs - 1) / runs);
     const dim3 grid(strips, (H + rows - 1) / rows);
-    const double e9 = 9.0 * eps * (F32IMG ? 1.0 : 255.0 * 255.0);
-    levin_sym_kernel<T, F32IMG, BANDS><<<grid, kAT, 0, st>>>(im, sc, e9, W, H, rows, o);
+    levin_sym_kernel<T, F32IMG, BANDS><<<grid, kAT, 0, st>>>(im, sc, ridge_for(eps, F32IMG), W, H, rows, o);
     GM_CUDA_TRY(cudaGetLastError());
     return GM_OK;
 }

@@ -197,3 +197,68 @@ def test_nonfinite_colours_stay_in_their_windows(orc, W, H, prec, bad):
             ok = np.isfinite(got)
             assert np.array_equal(ok, fin if name[0] == "w" else rows), (name, x, y)
             assert np.array_equal(got[ok], ref[ok]), (name, x, y)
+
+
+def _limit_couplings(image):
+    """Couplings (12, H, W) of whole-number colours (H, W, 3) for eps -> 0, FP64:
+    (1 + D_i^T N^+ D_j) / 9 per 3x3 window, N = 9 sum(x x^T) - S S^T, D = 9 x - S.  And the
+    smallest nonzero eigenvalue of any N."""
+    x = image.astype(np.float64)
+    H, W, _ = x.shape
+    win = np.stack([x[j:H - 2 + j, i:W - 2 + i] for j in range(3) for i in range(3)], axis=2)  # (h, w, 9, 3)
+    S = win.sum(2)
+    D = 9.0 * win - S[:, :, None, :]
+    N = 9.0 * np.einsum("hwqa,hwqb->hwab", win, win) - S[..., :, None] * S[..., None, :]  # whole numbers, exact
+    lam, vec = np.linalg.eigh(N)
+    real = lam > 1e-9 * np.maximum(lam[..., -1:], 1.0)
+    inv = np.where(real, 1.0 / np.where(real, lam, 1.0), 0.0)
+    y = np.einsum("hwqa,hwab->hwqb", D, vec)
+    t = (1.0 + np.einsum("hwpb,hwb,hwqb->hwpq", y, inv, y)) / 9.0
+    w = np.zeros((12, H, W))
+    for p in range(9):
+        for q in range(9):
+            k = (q % 3 - p % 3) + 5 * (q // 3 - p // 3)
+            if k > 0:
+                w[k - 1, p // 3:p // 3 + H - 2, p % 3:p % 3 + W - 2] += t[:, :, p, q]
+    return w, lam[real].min()
+
+
+@pytest.mark.parametrize("eps", [0.0, 1e-300, 1e-20])
+@pytest.mark.parametrize("prec,fmt", [("fp32", "rgb8"), ("fp16", "rgb8"), ("fp32", "rgba"), ("bf16", "rgba")])
+def test_assembly_of_singular_windows(prec, fmt, eps):
+    """eps = 0 and next to nothing on flat, white, black, grey, two-channel and
+    one-line patches (windows of rank 0, 1 and 2) beside noise: the limit of small
+    eps.  An addition of e to N moves the nine terms of a window by at most 8 e / lam
+    of the smallest nonzero eigenvalue lam; e is 2^-26 for bytes, and for floats
+    x = byte / 255 it is 9 2^-47 sum(x x) <= 243 2^-47, with three times that for the
+    rounding of the 24-bit colours' sums; FP32's rounding of the sum comes on top."""
+    torch = torch_cuda()
+    from gpumatting_b200 import api
+
+    W, H = 150, 40
+    rng = np.random.default_rng(5)
+    image = rng.integers(0, 256, size=(H, W, 3))
+    image[:, 20:32] = (77, 200, 30)
+    image[:, 32:44] = 255
+    image[:, 44:56] = 0
+    image[:, 60:76] = rng.integers(0, 256, size=(H, 16, 1))
+    image[:, 80:96, 2] = image[:, 80:96, 1]
+    image[:, 96:110, 0] = 9
+    image[:, 112:128] = (np.arange(16) * 3)[None, :, None]
+    image[:, 130:, 0] = 40
+    image[:, 130:, 1] = 41
+    want, lam = _limit_couplings(image)
+    img = torch.from_numpy(image.astype(np.uint8)).cuda()
+    e = 2.0 ** -26
+    if fmt == "rgba":
+        f = np.ones((H, W, 4), np.float32)
+        # bytes / 256: exact, so that windows have the ranks of the bytes' own
+        f[..., :3] = image / 256.0
+        img = torch.from_numpy(f).cuda()
+        e, lam = 3 * 243 * 2.0 ** -47, lam / 256.0 ** 2
+    st = api.LevinStore(W, H, prec).assemble(img, eps=eps)
+    got = st.planes("w32")[:, :, :W].double().cpu().numpy()
+    tol = np.spacing(np.abs(want).astype(np.float32)).astype(np.float64) + 9 * 8 * e / lam
+    assert np.all(np.abs(got - want) <= tol), np.nanmax(np.abs(got - want) / tol)
+    for n in ("w", "d", "d32"):
+        assert torch.isfinite(st.planes(n)[..., :W].float()).all()
