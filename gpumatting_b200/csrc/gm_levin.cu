@@ -140,7 +140,7 @@ struct SymOut {
 //
 // Measured with the FP16 store: 1080p RGB8 450 -> 114 us, 4096^2 4.3 -> 0.82 ms in a
 // row, 0.95-1.05 where another kernel's data has to leave L2 first (88 B written
-// per pixel are 28 and 225 us); FP32 store, 4001 x 2999: 2,400 -> 494 (RGB8), 556
+// per pixel are 28 and 225 us); FP32 store, 4001 x 2999: 2,400 -> 494 (RGB8), 550
 // us (float).  Bound by instruction issue at 12 warps per SM (about 60 % of the
 // slots, FP64 pipe 37 %).  Forms before: windows in shared memory 156 us
 // (12 shared wavefronts per 32 pixels and window); all rounded couplings through a
@@ -151,7 +151,7 @@ constexpr int kAP = kAT + 4;          // row length in shared memory (two pad co
 // CTAs per SM the registers are cut for.  A float image's 27 colours and 18 row
 // sums in 64 bits do not fit 168 registers (1080p: 160 us with 3 CTAs per SM, 135
 // with 2).  An RGB8 image's nearly do: 116 bytes a thread are spilled with a 2-byte
-// store (164 with the 25 bands), 8 with an FP32 one.  The 12 warps are worth
+// store (152 with the 25 bands), 8 with an FP32 one.  The 12 warps are worth
 // that: 122 us with 3 CTAs per SM and 135 with 2 before the diagonal's sums moved
 // to registers (4 bytes spilled then), 114 since.
 __host__ __device__ constexpr int asm_ctas(bool f32) { return f32 ? 2 : 3; }
@@ -215,14 +215,17 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
             if (kLowRing) lo[i / kAP][i % kAP] = T(0.f);
         }
 
-    // Colours (u - 1, u, u + 1) of row v, zero outside the image (and in an
-    // image without any window, whatever its colours hold): loaded for columns
-    // that are a window's centre, without a test for each (1080p FP16, RGB8 117 ->
-    // 114 us, float 134 -> 132).  A float image's for an FP32 store keep the tests:
-    // without them the kernel took 715 us instead of 556 at 4001 x 2999.
+    // Colours (u - 1, u, u + 1) of row v, zero outside the image and for columns
+    // that are no window's centre.  (The zero factors of a window outside the image
+    // do not make a float image's infinities and NaN zero: to the sides they are
+    // left out here, below the image the couplings they reach are cut.)  With an
+    // FP32 store a float image's three colours are loaded under a test each, which
+    // the middle one's, hidden from the compiler, keeps apart: as one block of loads
+    // they took the kernel from 562 to 715 us at 4001 x 2999 (550 this way).
     constexpr bool kByPixel = F32IMG && !kLow;
-    const bool in[3] = {u >= 1 && u <= W, u >= 0 && u < W, u >= -1 && u < W - 1};
-    const bool any = (kByPixel ? W >= 3 : ok_col) && H >= 3;
+    const bool any = (kByPixel || ok_col) && H >= 3;
+    int in[3] = {ok_col, ok_col, ok_col};
+    if (kByPixel) asm volatile("" : "+r"(in[1]));
     auto fetch = [&](int v, Pix (&p)[9]) {
 #pragma unroll
         for (int q = 0; q < 9; ++q) p[q] = 0;
@@ -362,6 +365,13 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
             }
             if (a == 1) p0[2] = pair(in0[2] + one, e, da[2]);
         }
+        if (F32IMG && r + 2 >= H) {  // couplings to rows below the image
+#pragma unroll
+            for (int n = 0; n < 9; ++n) {
+                p2[n] = 0.0;
+                if (r + 1 >= H) p1[n] = 0.0;
+            }
+        }
         // shares of the neighbouring columns' couplings: [9] planes, read from
         // t - 1 (0, 1, 4, 5) or t + 1 (2, 3, 6, 7, 8)
         xch[0][c] = p2[8]; xch[1][c] = p2[7]; xch[2][c] = p2[0]; xch[3][c] = p2[1];
@@ -400,11 +410,7 @@ __global__ void __launch_bounds__(kAT, asm_ctas(F32IMG)) levin_sym_kernel(ImgVie
         // x: column of the upper pixel less u; the lower one is du further, dv below
         auto finish = [&](int k, int x, double w9) {
             const int dv = (k + 2) / 5, du = k - 5 * dv;
-            // (a float image's infinities and NaN are not made zero by the zero
-            // factors of the windows outside it: couplings that leave it are cut)
-            const bool inside = !F32IMG || ((!kByPixel || x + du >= 0 || u >= 1) &&
-                                            (!kByPixel || x + du <= 0 || u + 1 < W) && (dv == 0 || r + dv < H));
-            const double w = inside ? w9 * (1.0 / 9.0) : 0.0;
+            const double w = w9 * (1.0 / 9.0);
             const float wf = __double2float_rn(w);
             const int row = ring_base(k) + (dv == 0 ? 0 : (dv == 1 ? r2 : r3));
             if (BANDS) hi[row][c + x] = wf;
